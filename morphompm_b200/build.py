@@ -21,7 +21,7 @@ LIB = os.path.join(OUT_DIR, "libmorphompm_b200.so")
 # the same sources with every kernel index checked (MPM_CHECK_BOUNDS)
 LIB_CHECKED = os.path.join(OUT_DIR, "libmorphompm_b200_checked.so")
 SOURCES = ["capi.cu"]
-HEADERS = ["mpm_common.cuh", "constitutive.cuh", "sort.cuh", "mpm_kernels.cuh"]
+HEADERS = ["mpm_common.cuh", "constitutive.cuh", "sort.cuh", "cluster_sort.cuh", "mpm_kernels.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -18,6 +18,7 @@
 #include "mpm_common.cuh"
 #include "constitutive.cuh"
 #include "sort.cuh"
+#include "cluster_sort.cuh"
 #include "mpm_kernels.cuh"
 
 using namespace mpm;
@@ -58,6 +59,9 @@ struct MpmPlan {
     size_t o_mkey = 0, o_mpart = 0, o_okey = 0, o_opart = 0, o_rint = 0, o_hist1 = 0;
     int nblk_sort1 = 1;     // blocks of the movers' radix sort (one key per thread)
     int nblk_resort = 1;
+    // one-launch sort of a small plan (cluster_sort.cuh): CTAs of its cluster
+    // (0: the general path), keys per thread, passes and digit bits
+    int cs_ctas = 0, cs_items = 1, cs_passes = 1, cs_bits = 1;
     char* chain_tape = nullptr;    // the tape whose sorted order the emitted mover flags refer to
     // runs of consecutive scenes with one material model (their slot ranges);
     // grouped: every model has one run, so each run gets a kernel for its model
@@ -117,8 +121,10 @@ Ctx make_ctx(MpmPlan* P) {
     c.ext_tau_bar = P->ext_tau_bar;
     c.dense_f = P->ws + P->o_dense_f;
     c.dense_b = P->ws + P->o_dense_b;
-    c.mover_flag = P->o_mflag == SIZE_MAX ? nullptr : at<unsigned char>(P, P->o_mflag);
-    c.mover_pflag = P->o_mflag == SIZE_MAX ? nullptr : at<unsigned char>(P, P->o_pflag);
+    // the cluster sort starts from the keys alone
+    const bool movers = P->o_mflag != SIZE_MAX && P->cs_ctas == 0;
+    c.mover_flag = movers ? at<unsigned char>(P, P->o_mflag) : nullptr;
+    c.mover_pflag = movers ? at<unsigned char>(P, P->o_pflag) : nullptr;
     c.n = P->n;
     c.n_tiles = P->n_tiles;
     c.n_keys = P->n_keys;
@@ -378,6 +384,70 @@ int run_resort(MpmPlan* P, const char* old_tape, char* tape, const unsigned* key
     return check_launch();
 }
 
+const void* cluster_sort_fn(int items) {
+    if (items == 8) return (const void*)cluster_sort_kernel<8>;
+    if (items == 4) return (const void*)cluster_sort_kernel<4>;
+    if (items == 2) return (const void*)cluster_sort_kernel<2>;
+    return (const void*)cluster_sort_kernel<1>;
+}
+
+cudaLaunchConfig_t cluster_sort_config(const MpmPlan* P, cudaLaunchAttribute* attr, cudaStream_t st) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)P->cs_ctas;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)P->cs_ctas);
+    cfg.blockDim = dim3(CS_THREADS);
+    cfg.dynamicSmemBytes = cluster_sort_smem(P->cs_items, P->cs_bits);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Shape of the cluster sort for this plan (0 CTAs: the general path).
+void plan_cluster_sort(MpmPlan* P) {
+    P->cs_ctas = 0;
+    if (P->n > CS_MAX_N || P->n_tiles > CS_MAX_TILES) return;
+    int ctas = 1, items = 1;
+    while (ctas < CS_MAX_CTAS && (long long)ctas * CS_THREADS < P->n) ctas *= 2;
+    while ((long long)ctas * CS_THREADS * items < P->n) items *= 2;
+    P->cs_ctas = ctas;
+    P->cs_items = items;
+    P->cs_passes = (P->key_bits + CS_MAX_BITS - 1) / CS_MAX_BITS;
+    P->cs_bits = (P->key_bits + P->cs_passes - 1) / P->cs_passes;
+}
+
+// Called with the plan's device current: the kernel's shared memory, and the
+// general path instead where the device cannot place the cluster.
+int bind_cluster_sort(MpmPlan* P) {
+    plan_cluster_sort(P);
+    if (P->cs_ctas == 0) return MPM_OK;
+    const void* fn = cluster_sort_fn(P->cs_items);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_sort_config(P, &attr, nullptr);
+    int clusters = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cluster_sort_smem(P->cs_items, CS_MAX_BITS)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        P->cs_ctas = 0;
+    }
+    return MPM_OK;
+}
+
+// keys -> sorted order, segment table and active-tile list in one launch
+int run_cluster_sort(MpmPlan* P, const Ctx& ctx, const unsigned* keys, unsigned* skeys, unsigned* perm, int* active,
+                     int* n_active, cudaStream_t st) {
+    Site site(P, MPM_K_SORT, 1, st);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_sort_config(P, &attr, st);
+    int* flag = ctx.tile_flag;
+    void* args[] = {(void*)&ctx, (void*)&keys, (void*)&skeys, (void*)&perm, (void*)&P->cs_passes, (void*)&P->cs_bits,
+                    (void*)&flag, (void*)&active, (void*)&n_active};
+    return cudaLaunchKernelExC(&cfg, cluster_sort_fn(P->cs_items), args) == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
+}
+
 // flags: MPM_FWD_CHAINED (keys and P2G records of `in` already formed by the
 // previous step's G2P), MPM_FWD_EMIT (form them for `out` in this G2P)
 template <typename R>
@@ -392,12 +462,16 @@ int step_fwd_R(MpmPlan* P, const MpmParticles& in, MpmParticles& out, int advect
     unsigned* keys = at<unsigned>(P, P->o_keys);
     R* payload = at<R>(P, P->o_payload);
     if (!chained) { Site s(P, MPM_K_BIN, 1, st); bin_kernel<R><<<g, B, 0, st>>>(ctx, in, keys); }
-    int rc = chained && P->chain_tape && ctx.mover_flag ? run_resort(P, P->chain_tape, tape, keys, st)
+    int rc;
+    if (P->cs_ctas > 0) {
+        rc = run_cluster_sort(P, ctx, keys, tp.skeys, tp.perm, tp.active, tp.n_active, st);
+        if (rc) return rc;
+    } else {
+        rc = chained && P->chain_tape && ctx.mover_flag ? run_resort(P, P->chain_tape, tape, keys, st)
                                                         : run_sort(P, keys, tp.skeys, tp.perm, st);
-    if (rc) return rc;
-    rc = build_segments(P, ctx, tp.skeys, st);
-    if (rc) return rc;
-    {
+        if (rc) return rc;
+        rc = build_segments(P, ctx, tp.skeys, st);
+        if (rc) return rc;
         Site s(P, MPM_K_COMPACT, 3, st);
         unsigned* tblk = at<unsigned>(P, P->o_tblk);
         tile_count_kernel<<<P->nblk_tile, SEG_THREADS, 0, st>>>(ctx.tile_flag, P->n_tiles, tblk);
@@ -745,6 +819,7 @@ int mpm_plan_bind(MpmPlan* P, void* workspace, void* stream) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return MPM_ERR_CUDA;
     cudaDeviceGetAttribute(&P->n_sm, cudaDevAttrMultiProcessorCount, dev);
+    if (int rc = bind_cluster_sort(P)) return rc;
     if (cudaMemcpyAsync(P->ws + P->o_scenes, P->scenes.data(), sizeof(MpmScene) * P->scenes.size(),
                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(P->ws + P->o_aux, P->aux.data(), sizeof(SceneAux) * P->aux.size(),
