@@ -98,8 +98,8 @@ typedef struct MpmCotangents {
 /* Schedule knobs (picked by the autotuner; zeros select the defaults). */
 typedef struct MpmTuning {
     int32_t tile_xy;             /* node tile edge in x and y: 4, 8 or 16 (default 4)       */
-    int32_t scatter_ctas_per_sm; /* persistent P2G node-gather grid = SMs x this (1024-thread CTAs, default 1) */
-    int32_t scatter_oxb;         /* stencil x-offsets per pass: 3 (FP32 default) or 1       */
+    int32_t scatter_ctas_per_sm; /* P2G node-gather grid: at most 16 blocks of 128 threads per SM x this (default 1) */
+    int32_t scatter_oxb;         /* accepted, without effect: three lanes per cell take the three x-offsets */
     int32_t particle_block;      /* threads per block of the per-particle kernels: 64, 128 or 256 (default) */
     int32_t active_tile_cap;     /* capacity of the active-tile list (0 = every tile)       */
     float fp64_gap_thresh;       /* FP32 Hencky: relative singular-value gap below this is

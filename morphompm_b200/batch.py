@@ -7,8 +7,7 @@ adjoint trajectory is captured once in a CUDA graph and replayed.  Growth is
 the per-scene isotropic law Fg = g_s I (growth_mode 1, g_s = 1 + A_s), so the
 adjoint returns d loss / d g_s per scene, accumulated in float64.
 
-The schedule (node-tile edge, P2G CTAs per SM, stencil offsets per pass,
-particle block size) is chosen by ``autotune``, which times short forward
+The schedule (node-tile edge, P2G CTAs per SM, particle block size) is chosen by ``autotune``, which times short forward
 trajectories of the actual batch for each candidate on the current GPU.
 """
 from __future__ import annotations
@@ -292,7 +291,6 @@ CANDIDATES = {
     "tile_xy": [4, 8],
     "tile_z": [4, 8, 16],
     "scatter_ctas_per_sm": [1, 2],
-    "scatter_oxb": [1, 3],
     "particle_block": [128, 256],
 }
 TUNE_CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned.json")
@@ -347,8 +345,6 @@ def autotune(scenes: List[dict], dtype=torch.float32, steps: int = 4, budget_s: 
         for v in vals:
             if time.time() - t_start > budget_s:
                 break
-            if dtype == torch.float64 and knob == "scatter_oxb" and v == 3:
-                continue
             cfg = dict(best, **{knob: v})
             key = json.dumps(cfg, sort_keys=True)
             if key in results:

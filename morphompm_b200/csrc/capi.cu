@@ -51,7 +51,7 @@ struct MpmPlan {
     int TN = 0, active_cap = 0;
     bool any_growth = false;
     // workspace offsets
-    size_t o_scenes, o_aux, o_scene_of, o_tile_scene, o_status, o_cell_seg, o_blk, o_tblk;
+    size_t o_scenes, o_aux, o_sk, o_scene_of, o_tile_scene, o_status, o_cell_seg, o_blk, o_tblk;
     size_t o_tile_flag, o_keys, o_kalt0, o_valt0, o_kalt1, o_valt1, o_hist, o_totals, o_payload, o_sums;
     size_t o_dense_f = 0, o_dense_b = 0;
     // incremental re-sort of chained steps (SIZE_MAX: not laid out)
@@ -104,6 +104,7 @@ Ctx make_ctx(MpmPlan* P) {
     Ctx c;
     c.scenes = at<const MpmScene>(P, P->o_scenes);
     c.aux = at<const SceneAux>(P, P->o_aux);
+    c.sk = P->ws + P->o_sk;
     c.scene_of = at<const int>(P, P->o_scene_of);
     c.tile_scene = at<const int>(P, P->o_tile_scene);
     c.status = at<int>(P, P->o_status);
@@ -201,6 +202,22 @@ inline int check_launch() {
     return e == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
 
+// The scenes' constants in the plan's real type -> workspace.  `host` must stay
+// valid until the copy has run.
+int upload_scene_constants(MpmPlan* P, std::vector<char>& host, cudaStream_t st) {
+    const size_t S = P->scenes.size(), each = P->real_bytes == 4 ? sizeof(SceneK<float>) : sizeof(SceneK<double>);
+    host.resize(S * each);
+    for (size_t i = 0; i < S; ++i) {
+        if (P->real_bytes == 4)
+            reinterpret_cast<SceneK<float>*>(host.data())[i] = scene_constants<float>(P->scenes[i]);
+        else
+            reinterpret_cast<SceneK<double>*>(host.data())[i] = scene_constants<double>(P->scenes[i]);
+    }
+    return cudaMemcpyAsync(P->ws + P->o_sk, host.data(), host.size(), cudaMemcpyHostToDevice, st) == cudaSuccess
+               ? MPM_OK
+               : MPM_ERR_CUDA;
+}
+
 // segment table of the sorted keys (and, in the forward, the active tile flags)
 int build_segments(MpmPlan* P, const Ctx& ctx, const unsigned* skeys, cudaStream_t st) {
     Site site(P, MPM_K_MARK, 3, st);
@@ -208,14 +225,6 @@ int build_segments(MpmPlan* P, const Ctx& ctx, const unsigned* skeys, cudaStream
     scan_counts_kernel<<<1, 1024, 0, st>>>(ctx.blk_count, P->nblk_seg, ctx.n_seg, INT_MAX, ctx.status);
     seg_write_kernel<<<P->nblk_seg, SEG_THREADS, 0, st>>>(ctx, skeys);
     return check_launch();
-}
-
-template <typename R, int MODE>
-void* sums_fn(int oxb) {
-    if constexpr (sizeof(R) == 4) {
-        if (oxb == 3) return (void*)cell_sums_kernel<R, MODE, 3>;
-    }
-    return (void*)cell_sums_kernel<R, MODE, 1>;
 }
 
 template <typename R, int T, int MODE>
@@ -236,30 +245,28 @@ template <typename R>
 int launch_nodes(MpmPlan* P, int mode, const Ctx& ctx, const int* active, const int* nact, R* grid_out,
                  const R* grid_fwd, int advect, cudaStream_t st) {
     const R* Sc = at<R>(P, P->o_sums);
-    long long cap = P->n;
-    int ctas = P->n_sm * std::max(1, P->tune.scatter_ctas_per_sm);
-    ctas = std::max(1, std::min(ctas, P->active_cap));
+    // blocks for every node the tape's tile list can hold, at most two waves of them
+    const long long need = ((long long)P->active_cap * P->TN + NODE_THREADS - 1) / NODE_THREADS;
+    const long long room = (long long)P->n_sm * 16 * std::max(1, P->tune.scatter_ctas_per_sm);
+    const int ctas = (int)std::max<long long>(1, std::min<long long>(need, room));
     void* f2 = mode == 0 ? nodes_fn<R, 0>(P->tune.tile_xy, P->tune.tile_z)
                          : nodes_fn<R, 1>(P->tune.tile_xy, P->tune.tile_z);
-    void* a2[] = {(void*)&ctx, (void*)&Sc, (void*)&cap, (void*)&active, (void*)&nact, (void*)&grid_out,
+    void* a2[] = {(void*)&ctx, (void*)&Sc, (void*)&active, (void*)&nact, (void*)&grid_out,
                   (void*)&grid_fwd, (void*)&advect};
-    return cudaLaunchKernel(f2, dim3(ctas), dim3(1024), a2, 0, st) == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
+    return cudaLaunchKernel(f2, dim3(ctas), dim3(NODE_THREADS), a2, 0, st) == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
 
-// two-phase P2G: per-cell stencil sums, then per-node gather + grid epilogue
-template <typename R>
-int launch_p2g(MpmPlan* P, int mode, const Ctx& ctx, const unsigned* perm, const R* payload, const int* active,
-               const int* nact,
-               R* grid_out, const R* grid_fwd, int advect, cudaStream_t st) {
-    R* S = at<R>(P, P->o_sums);
-    long long cap = P->n;
-    int blocks1 = (int)std::min<long long>((P->n + 127) / 128, (long long)P->n_sm * 16);
-    blocks1 = std::max(1, blocks1);
-    void* f1 = mode == 0 ? sums_fn<R, 0>(P->tune.scatter_oxb) : sums_fn<R, 1>(P->tune.scatter_oxb);
-    void* a1[] = {(void*)&ctx, (void*)&perm, (void*)&payload, (void*)&S, (void*)&cap};
-    if (cudaLaunchKernel(f1, dim3(blocks1), dim3(128), a1, 0, st) != cudaSuccess) return MPM_ERR_CUDA;
-    P->launches += 1;   // the Site around this call counts one
-    return launch_nodes<R>(P, mode, ctx, active, nact, grid_out, grid_fwd, advect, st);
+// P2G phase 1 (per-cell stencil sums): forward from the P2G records, ADJ from
+// the output cotangents.  One warp per CS_CELLS segments of a device-side
+// count, at most n of them.
+template <typename R, bool ADJ>
+int launch_cells(MpmPlan* P, const Ctx& ctx, const Tape<R>& tp, const R* payload, const MpmParticles& in,
+                 const MpmCotangents& ob, int advect, cudaStream_t st) {
+    constexpr int W = CellSums<R>::WARPS;
+    const long long blocks = std::min<long long>((P->n + W * CS_CELLS - 1) / (W * CS_CELLS), (long long)P->n_sm * 64);
+    cell_sums_kernel<R, ADJ><<<(int)std::max<long long>(1, blocks), 32 * W, 0, st>>>(
+        ctx, tp.skeys, tp.perm, payload, in, ob, at<R>(P, P->o_sums), advect);
+    return check_launch();
 }
 
 // Stable LSD radix sort of kin (with payload vin, or the index when null)
@@ -483,8 +490,10 @@ int step_fwd_R(MpmPlan* P, const MpmParticles& in, MpmParticles& out, int advect
     rc = check_launch();
     if (rc) return rc;
     {
-        Site s(P, MPM_K_P2G, 1, st);
-        rc = launch_p2g<R>(P, 0, ctx, tp.perm, payload, tp.active, tp.n_active, tp.grid, nullptr, advect, st);
+        Site s(P, MPM_K_P2G, 2, st);
+        rc = launch_cells<R, false>(P, ctx, tp, payload, in, MpmCotangents{}, advect, st);
+        if (rc) return rc;
+        rc = launch_nodes<R>(P, 0, ctx, tp.active, tp.n_active, tp.grid, nullptr, advect, st);
     }
     if (rc) return rc;
     {
@@ -510,25 +519,10 @@ int step_bwd_R(MpmPlan* P, const MpmParticles& in, const void* outC, const MpmCo
     const int B = P->tune.particle_block;
     const int g = grid_for(P->n, B);
     double* dbuf = at<double>(P, P->o_dbuf);
-    {
-        // the forward step's segment table is in the tape: restore the cell marks
-        Site s(P, MPM_K_MARK, 1, st);
-        const int blocks = (int)std::max<long long>(1, std::min<long long>((P->n + 255) / 256, (long long)P->n_sm * 8));
-        remark_cells_kernel<<<blocks, 256, 0, st>>>(ctx, tp.skeys);
-    }
-    int rc = check_launch();
-    if (rc) return rc;
+    int rc;
     {
         Site s(P, MPM_K_BWD_P2G, 2, st);
-        R* S = at<R>(P, P->o_sums);
-        long long cap = P->n;
-        int blocks1 = (int)std::min<long long>((P->n + 127) / 128, (long long)P->n_sm * 16);
-        blocks1 = std::max(1, blocks1);
-        if (P->tune.scatter_oxb == 3 && sizeof(R) == 4)
-            cell_sums_adj_kernel<R, 3><<<blocks1, 128, 0, st>>>(ctx, tp.perm, in, ob, S, cap, advect);
-        else
-            cell_sums_adj_kernel<R, 1><<<blocks1, 128, 0, st>>>(ctx, tp.perm, in, ob, S, cap, advect);
-        rc = check_launch();
+        rc = launch_cells<R, true>(P, ctx, tp, nullptr, in, ob, advect, st);
         if (rc) return rc;
         rc = launch_nodes<R>(P, 1, ctx, tp.active, tp.n_active, nullptr, tp.grid, advect, st);
     }
@@ -624,8 +618,6 @@ int mpm_plan_create(const MpmScene* scenes, int32_t n_scenes, int32_t real_bytes
     if (P->tune.tile_xy != 8 && P->tune.tile_xy != 16) P->tune.tile_xy = 4;
     if (P->tune.tile_z != 8 && P->tune.tile_z != 16) P->tune.tile_z = 4;
     if (P->tune.scatter_ctas_per_sm <= 0) P->tune.scatter_ctas_per_sm = 1;
-    if (P->tune.scatter_oxb != 1 && P->tune.scatter_oxb != 3) P->tune.scatter_oxb = real_bytes == 4 ? 3 : 1;
-    if (real_bytes == 8) P->tune.scatter_oxb = 1;
     // the per-particle kernels are compiled for at most 256 threads per block
     if (P->tune.particle_block != 64 && P->tune.particle_block != 128) P->tune.particle_block = 256;
     if (P->tune.fp64_gap_thresh == 0.0f) P->tune.fp64_gap_thresh = 1e-6f;
@@ -702,6 +694,7 @@ int mpm_plan_create(const MpmScene* scenes, int32_t n_scenes, int32_t real_bytes
     Layout L;
     P->o_scenes = L.take(sizeof(MpmScene) * P->scenes.size());
     P->o_aux = L.take(sizeof(SceneAux) * P->aux.size());
+    P->o_sk = L.take((real_bytes == 4 ? sizeof(SceneK<float>) : sizeof(SceneK<double>)) * P->scenes.size());
     P->o_scene_of = L.take(n * 4);
     P->o_tile_scene = L.take(nt * 4);
     P->o_status = L.take(128);
@@ -719,7 +712,7 @@ int mpm_plan_create(const MpmScene* scenes, int32_t n_scenes, int32_t real_bytes
     P->o_hist = L.take((size_t)RADIX * P->nblk_sort * 4);
     P->o_totals = L.take(RADIX * 4);
     P->o_payload = L.take(n * PAYLOAD * R);
-    P->o_sums = L.take(27 * n * 4 * R);
+    P->o_sums = L.take((size_t)sum_entries(P->n) * 4 * R);
     P->o_dense_f = L.take((size_t)P->n_nodes * 4 * R);
     P->o_dense_b = L.take((size_t)P->n_nodes * 4 * R);
     P->o_dbuf = L.take(3 * n * 8);      // dL/dA, dL/dmu, dL/dlambda per slot
@@ -820,6 +813,8 @@ int mpm_plan_bind(MpmPlan* P, void* workspace, void* stream) {
     if (cudaGetDevice(&dev) != cudaSuccess) return MPM_ERR_CUDA;
     cudaDeviceGetAttribute(&P->n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (int rc = bind_cluster_sort(P)) return rc;
+    std::vector<char> sk;
+    if (int rc = upload_scene_constants(P, sk, st)) return rc;
     if (cudaMemcpyAsync(P->ws + P->o_scenes, P->scenes.data(), sizeof(MpmScene) * P->scenes.size(),
                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(P->ws + P->o_aux, P->aux.data(), sizeof(SceneAux) * P->aux.size(),
@@ -865,7 +860,9 @@ int mpm_plan_update_scenes(MpmPlan* P, const MpmScene* scenes, int32_t n_scenes,
     for (int s = 0; s < n_scenes; ++s) P->scenes[s] = scenes[s];
     P->chain_valid = false;     // records formed with the old parameters
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemcpyAsync(P->ws + P->o_scenes, P->scenes.data(), sizeof(MpmScene) * P->scenes.size(),
+    std::vector<char> sk;
+    if (upload_scene_constants(P, sk, st) != MPM_OK ||
+        cudaMemcpyAsync(P->ws + P->o_scenes, P->scenes.data(), sizeof(MpmScene) * P->scenes.size(),
                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return MPM_ERR_CUDA;
@@ -1251,7 +1248,10 @@ int mpm_loss_mse(MpmPlan* P, const void* x, int64_t sp3, int64_t sc3, const void
 // ---------------------------------------------------------------------------
 namespace {
 
-__device__ __align__(256) unsigned char g_noalloc_scratch[MPM_NOALLOC_SCRATCH_BYTES];
+// The limit a scene must fit counts 27 n entries of cell sums; the blocked
+// layout rounds n up to whole blocks, for which the array has room beyond it.
+constexpr size_t NOALLOC_EXTRA = (size_t)27 * SUM_BLOCK * 4 * 8;
+__device__ __align__(256) unsigned char g_noalloc_scratch[MPM_NOALLOC_SCRATCH_BYTES + NOALLOC_EXTRA];
 
 constexpr int NOALLOC_MAX_DEVICES = 64;
 struct NoallocDevice {
@@ -1320,6 +1320,8 @@ int noalloc_scratch(void** out, int* n_sm) {
     return MPM_OK;
 }
 
+constexpr size_t NOALLOC_SK = (sizeof(SceneAux) + 15) / 16 * 16;
+
 // Forward-only workspace layout of one scene (the fields step_fwd_R reads),
 // on a plan object that owns no heap memory.
 bool noalloc_layout(MpmPlan& P, const MpmScene& sc, int real_bytes, SceneAux& a) {
@@ -1327,7 +1329,6 @@ bool noalloc_layout(MpmPlan& P, const MpmScene& sc, int real_bytes, SceneAux& a)
     P.tune.tile_xy = 4;
     P.tune.tile_z = 4;
     P.tune.scatter_ctas_per_sm = 1;
-    P.tune.scatter_oxb = real_bytes == 4 ? 3 : 1;
     P.tune.particle_block = 256;
     P.tune.fp64_gap_thresh = 1e-6f;
     const int T = P.tune.tile_xy, TZ = P.tune.tile_z;
@@ -1366,7 +1367,10 @@ bool noalloc_layout(MpmPlan& P, const MpmScene& sc, int real_bytes, SceneAux& a)
     P.tape_bytes = tl.off;
     Layout L;
     P.o_scenes = L.take(sizeof(MpmScene));
-    P.o_aux = L.take(sizeof(SceneAux));
+    // the aux entry and the scene constants share one aligned block
+    static_assert(NOALLOC_SK + sizeof(SceneK<double>) <= ALIGN, "scene constants after the aux entry");
+    P.o_aux = L.take(NOALLOC_SK + sizeof(SceneK<double>));
+    P.o_sk = P.o_aux + NOALLOC_SK;
     P.o_scene_of = L.take(n * 4);
     P.o_tile_scene = L.take(nt * 4);
     P.o_status = L.take(128);
@@ -1383,12 +1387,13 @@ bool noalloc_layout(MpmPlan& P, const MpmScene& sc, int real_bytes, SceneAux& a)
     P.o_hist = L.take((size_t)RADIX * P.nblk_sort * 4);
     P.o_totals = L.take(RADIX * 4);
     P.o_payload = L.take(n * PAYLOAD * R);
-    P.o_sums = L.take(27 * n * 4 * R);
+    P.o_sums = L.take((size_t)sum_entries(P.n) * 4 * R);
     P.o_dense_f = L.take((size_t)P.n_nodes * 4 * R);
     P.o_dense_b = P.o_dense_f;      // the forward step writes no reverse records
     P.o_tape = L.take(P.tape_bytes);
     P.ws_bytes = L.off;
-    return P.ws_bytes <= (size_t)MPM_NOALLOC_SCRATCH_BYTES;
+    const size_t rounded = align_up((size_t)sum_entries(P.n) * 4 * R) - align_up(27 * n * 4 * R);
+    return P.ws_bytes - rounded <= (size_t)MPM_NOALLOC_SCRATCH_BYTES;
 }
 
 }  // namespace
@@ -1412,8 +1417,13 @@ extern "C" int mpm_step_fwd_noalloc(const MpmScene* scene, int32_t real_bytes, c
     P.ws = static_cast<char*>(ws);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // the scene tables, and everything the step expects to start at zero
+    const SceneK<float> skf = scene_constants<float>(*scene);
+    const SceneK<double> skd = scene_constants<double>(*scene);
     if (cudaMemcpyAsync(P.ws + P.o_scenes, scene, sizeof(MpmScene), cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(P.ws + P.o_aux, &aux, sizeof(SceneAux), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        (real_bytes == 4
+             ? cudaMemcpyAsync(P.ws + P.o_sk, &skf, sizeof(skf), cudaMemcpyHostToDevice, st)
+             : cudaMemcpyAsync(P.ws + P.o_sk, &skd, sizeof(skd), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         cudaMemsetAsync(P.ws + P.o_scene_of, 0, (size_t)P.n * 4, st) != cudaSuccess ||
         cudaMemsetAsync(P.ws + P.o_tile_scene, 0, (size_t)P.n_tiles * 4, st) != cudaSuccess ||
         cudaMemsetAsync(P.ws + P.o_status, 0, 128, st) != cudaSuccess ||

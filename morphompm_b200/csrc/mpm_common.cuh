@@ -50,10 +50,43 @@ struct SceneAux {
     int ncells;             // (shape+2)^3 padded cells; key cell_begin+ncells = "outside"
 };
 
+// Scene constants in the plan's real type, converted (and the reciprocal of dx
+// formed in FP64) once on the host: a per-particle kernel would spend about 60
+// instructions on the FP64 division and the conversions.
+template <typename R>
+struct SceneK {
+    R dx, dt, inv_dx, pmass, vol0;
+    R s_damp, mass_eps, gravity[3];     // s_damp = 1 - damping
+    int shape[3];
+    int growth_mode;
+    int wall, clamp_lo[3], clamp_hi[3];
+};
+template <typename R>
+inline SceneK<R> scene_constants(const MpmScene& sc) {
+    SceneK<R> k;
+    k.dx = (R)sc.dx;
+    k.dt = (R)sc.dt;
+    k.inv_dx = (R)(1.0 / sc.dx);
+    k.pmass = (R)sc.pmass;
+    k.vol0 = (R)sc.vol0;
+    k.s_damp = (R)(1.0 - sc.damping);
+    k.mass_eps = (R)sc.mass_eps;
+    for (int d = 0; d < 3; ++d) {
+        k.gravity[d] = (R)sc.gravity[d];
+        k.shape[d] = sc.shape[d];
+        k.clamp_lo[d] = sc.clamp_lo[d];
+        k.clamp_hi[d] = sc.clamp_hi[d];
+    }
+    k.growth_mode = sc.growth_mode;
+    k.wall = sc.wall;
+    return k;
+}
+
 // Workspace pointers and sizes, passed by value to every kernel.
 struct Ctx {
     const MpmScene* scenes;
     const SceneAux* aux;
+    const void* sk;              // SceneK<real> of each scene
     const int* scene_of;         // scene of each particle slot (same ranges sorted or not)
     const int* tile_scene;       // scene of each tile
     int* status;                 // device status word (MPM_* bits)

@@ -2,26 +2,31 @@
 //
 // Forward (python/morphompm/transfer.py:33-79):
 //   bin_kernel        cell key of every particle (stencil base, exact rounding)
+//   cluster sort      (cluster_sort.cuh) small plans: sorted order, segments and
+//                     active tiles in one launch, instead of the next three
 //   radix sort        (sort.cuh) cell-sorted particle order, deterministic
 //   seg_* kernels     segment table of the occupied cells + active tile flags
 //   compact_tiles     active node tiles -> compact grid slots
 //   prepass_kernel    stress and the P2G record of every particle (particle order);
 //                     in a chain of steps the previous G2P forms them instead
-//   cell_sums_kernel  P2G phase 1: per occupied cell, its 27 stencil sums
+//   cell_sums_kernel  P2G phase 1: per occupied cell, its 27 stencil sums, from
+//                     records staged in shared memory
 //   node_sums_kernel  P2G phase 2: per node, the sums of its 27 source cells
 //                     in a fixed order, + grid update with boundary conditions
 //   g2p_kernel        gather, advect, F update; clears the cell marks; in a
 //                     chain also bins the new state and forms its P2G records
 // Reverse (python/morphompm/transfer.py:82-158):
-//   cell_sums_adj     gv_b scatter phase 1 (nv_b, Cn_b' formed per particle)
+//   cell_sums<ADJ>    gv_b scatter phase 1 (nv_b, Cn_b' formed per particle)
 //   node_sums<1>      gv_b gather + grid adjoint (gmom_b, gm_b)
 //   bwd_particle_kernel  P2G adjoint, constitutive VJP, volume path, x_b terms
 //
 // P2G determinism: particles are sorted by cell, every occupied cell's sums
-// are formed by one thread in sorted particle order, and every node adds its
+// are formed in sorted particle order (one thread per x-offset of the stencil), and every node adds its
 // source cells in the fixed order of the stencil offsets.  No atomics, no
 // shared-memory races: the result does not depend on scheduling.
 #pragma once
+
+#include <limits.h>
 
 #include "mpm_common.cuh"
 #include "constitutive.cuh"
@@ -83,7 +88,8 @@ __device__ __forceinline__ void store_node(R* __restrict__ g, long long idx, con
     }
 }
 
-__device__ __forceinline__ bool node_free(const MpmScene& sc, int i, int j, int k) {
+template <typename R>
+__device__ __forceinline__ bool node_free(const SceneK<R>& sc, int i, int j, int k) {
     if (sc.wall > 0) {
         int w = sc.wall;
         if (i < w || j < w || k < w || i >= sc.shape[0] - w || j >= sc.shape[1] - w || k >= sc.shape[2] - w)
@@ -309,30 +315,6 @@ scan_counts_kernel(unsigned* __restrict__ cnt, int nblk, int* __restrict__ total
     }
 }
 
-// Reverse step: the segment table is the one the forward step recorded in the
-// tape; only the dense cell marks (cleared by the forward G2P) are restored.
-__global__ void __launch_bounds__(256)
-remark_cells_kernel(Ctx ctx, const unsigned* __restrict__ skeys) {
-    const int nseg = *ctx.n_seg;
-    // NB segments per thread and pass, their loads issued together
-    constexpr int NB = 4;
-    const int stride = gridDim.x * blockDim.x;
-    for (int id0 = blockIdx.x * blockDim.x + threadIdx.x; id0 < nseg; id0 += NB * stride) {
-        int f[NB];
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int id = id0 + b * stride;
-            f[b] = id < nseg ? ctx.seg_first[id] : -1;
-        }
-        unsigned k[NB];
-#pragma unroll
-        for (int b = 0; b < NB; ++b) k[b] = (f[b] >= 0 && MPM_INB(f[b], ctx.n, 11)) ? skeys[f[b]] : 0xffffffffu;
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-            if (f[b] >= 0 && k[b] != 0xffffffffu && MPM_INB(k[b], ctx.n_keys, 2)) ctx.cell_seg[k[b]] = id0 + b * stride + 1;
-    }
-}
-
 // exclusive scan, in place, of a block's E (round, warp) counts (round-major;
 // warp 0, E / 32 per lane, or one per lane for E <= 32); call from all threads
 template <int E>
@@ -518,12 +500,26 @@ prepass_kernel(Ctx ctx, MpmParticles P, R* __restrict__ payload, int t) {
 }
 
 // ---------------------------------------------------------------------------
-// P2G, phase 1: per-cell sums.  One thread per segment (occupied cell) adds
-// its particles' contributions to the 27 stencil nodes, in sorted order, in
-// registers, and stores them as sums[o][segment] (o = 9 ox + 3 oy + oz).
-// MODE 0: channels (m, mom[3]);  MODE 1: channels (gv_b[3], unused).
-// OXB: stencil x-offsets accumulated per pass over the cell's particles.
+// P2G, phase 1: per-cell sums.  For every segment (occupied cell) the sums of
+// its particles' contributions to the 27 stencil nodes, in sorted order,
+// stored at sum_at(o, segment) (o = 9 ox + 3 oy + oz).
+// Forward: channels (m, mom[3]), from the P2G records.
+// ADJ (transfer.py:99-119, the scatter of gv_b): w (nv_b + k4 Cn_b' dp), with
+// nv_b = vn_b + dt xn_b (advect) and Cn_b' = Cn_b + dt Fn_b F^T formed here
+// from the cotangents of the step's output; the cell marks, cleared by the
+// forward G2P, are restored for the node gather.
 // ---------------------------------------------------------------------------
+// Entry of stencil offset o of segment id in the sums: blocks of SUM_BLOCK
+// segments hold their 27 offsets together, so that the entries that a warp
+// touches lie in a few kilobytes and not in 27 arrays of n entries.
+constexpr int SUM_BLOCK = 32;
+__host__ __device__ __forceinline__ long long sum_at(int o, int id) {
+    return ((long long)(id / SUM_BLOCK) * 27 + o) * SUM_BLOCK + id % SUM_BLOCK;
+}
+__host__ __device__ __forceinline__ long long sum_entries(long long n) {
+    return (n + SUM_BLOCK - 1) / SUM_BLOCK * SUM_BLOCK * 27;
+}
+
 template <typename R>
 __device__ __forceinline__ void store_sum(R* __restrict__ S, long long idx, const R v[4]) {
     if constexpr (sizeof(R) == 4) {
@@ -535,197 +531,210 @@ __device__ __forceinline__ void store_sum(R* __restrict__ S, long long idx, cons
     }
 }
 
-// Adds one particle record's contributions to the stencil sums of the x-offsets
-// ox0 .. ox0+OXB-1: w(o) (a + B dp(o)) (and w(o) m in channel 0 for MODE 0),
-// dp = o - fx in cell units (B carries the dx factor).
-template <typename R, int MODE, int OXB>
-__device__ __forceinline__ void accumulate_record(const R r[PAYLOAD], int ox0, R acc[OXB][3][3][4]) {
-    R w[3][3];
-    bspline(r, w);
-    R dz[3] = {R(0) - r[2], R(1) - r[2], R(2) - r[2]};
-    R dy[3] = {R(0) - r[1], R(1) - r[1], R(2) - r[1]};
+// What bounds it: with one thread per cell every load touched 32 sectors, and
+// a cell's particles were re-read from L2 (FP64: in three passes of the
+// registers' choosing).  On 4.7M FP32 particles the reverse took 284 us and the
+// forward 166, now 224 and 145; on 0.76M FP64 particles 529 and 93, now 80 and
+// 61; on 4096 FP64 particles 33 and 18, now 6.4 and 5.4.  At 4.7M it moves its
+// 0.95 GB (reverse) at 4.2 TB/s; the rest is the wait between a warp's loading
+// and adding (45% of the issue slots used).
+//
+// A warp takes CS_CELLS consecutive segments, whose particles are consecutive
+// sorted slots.  Its lanes first bring the particles' records into shared
+// memory, one particle per lane (every load coalesced), at most CS_SLOTS slots
+// at a time; then three lanes per cell, one per stencil x-offset, add them up
+// in sorted order.  CS_STRIDE: reals per record in shared memory, 16 padded so
+// that the 16-byte accesses of consecutive slots fall on distinct banks.
+// MIN_CTAS: registers for a round's loads in flight come before more warps
+// (FP64 reverse 105 us with 5 CTAs per SM, 80 with 4; FP32 on (n, 3, 3) fields
+// 103 with 6, 85 with 5, and on rows of n 231 with 6, 224 with 5, 239 with 4).
+constexpr int CS_CELLS = 10;
+constexpr int CS_SLOTS = 96;
+template <typename R> struct CellSums;
+template <> struct CellSums<float>  { static constexpr int WARPS = 4, STRIDE = 20, MIN_CTAS = 5; };
+template <> struct CellSums<double> { static constexpr int WARPS = 3, STRIDE = 18, MIN_CTAS = 4; };
+
+// Offset of a slot's record.  Another 16 bytes after every 8 slots: with 8
+// particles per cell the ten cells' lanes read slots 8 apart, which would
+// otherwise all start on the same bank.
+template <typename R>
+__host__ __device__ constexpr int rec_at(int slot) {
+    return slot * CellSums<R>::STRIDE + (slot >> 3) * (int)(16 / sizeof(R));
+}
+
+template <typename R>
+__device__ __forceinline__ void put_record(R* at, const R r[PAYLOAD]) {
+    using V = typename Vec4<R>::T;
+    constexpr int per = sizeof(V) / sizeof(R);
 #pragma unroll
-    for (int a = 0; a < OXB; ++a) {
-        const int ox = ox0 + a;
-        const R dpx = R(ox) - r[0];
-        R wx;
-        if constexpr (OXB == 3) wx = w[a][0];
-        else wx = ox == 0 ? w[0][0] : (ox == 1 ? w[1][0] : w[2][0]);
-        // a + B dp with dp = (dpx, dy, dz), x part hoisted
-        const R ax0 = r[4] + r[7] * dpx, ax1 = r[5] + r[10] * dpx, ax2 = r[6] + r[13] * dpx;
+    for (int i = 0; i < PAYLOAD / per; ++i) reinterpret_cast<V*>(at)[i] = reinterpret_cast<const V*>(r)[i];
+}
+template <typename R>
+__device__ __forceinline__ void get_record(const R* at, R r[PAYLOAD]) {
+    using V = typename Vec4<R>::T;
+    constexpr int per = sizeof(V) / sizeof(R);
 #pragma unroll
-        for (int oy = 0; oy < 3; ++oy) {
-            const R wxy = wx * w[oy][1];
-            const R ay0 = ax0 + r[8] * dy[oy], ay1 = ax1 + r[11] * dy[oy], ay2 = ax2 + r[14] * dy[oy];
+    for (int i = 0; i < PAYLOAD / per; ++i) {
+        const V v = reinterpret_cast<const V*>(at)[i];
+        const R* e = reinterpret_cast<const R*>(&v);
 #pragma unroll
-            for (int oz = 0; oz < 3; ++oz) {
-                const R wt = wxy * w[oz][2];
-                const R q0 = ay0 + r[9] * dz[oz];
-                const R q1 = ay1 + r[12] * dz[oz];
-                const R q2 = ay2 + r[15] * dz[oz];
-                if constexpr (MODE == 0) {
-                    acc[a][oy][oz][0] += wt * r[3];
-                    acc[a][oy][oz][1] += wt * q0;
-                    acc[a][oy][oz][2] += wt * q1;
-                    acc[a][oy][oz][3] += wt * q2;
-                } else {
-                    acc[a][oy][oz][0] += wt * q0;
-                    acc[a][oy][oz][1] += wt * q1;
-                    acc[a][oy][oz][2] += wt * q2;
-                }
-            }
-        }
+        for (int k = 0; k < per; ++k) r[i * per + k] = e[k];
     }
 }
 
-template <typename R, int OXB>
-__device__ __forceinline__ void zero_acc(R acc[OXB][3][3][4]) {
-#pragma unroll
-    for (int a = 0; a < OXB; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int h = 0; h < 4; ++h) acc[a][b][c][h] = R(0);
-}
-
-template <typename R, int OXB>
-__device__ __forceinline__ void store_acc(R* __restrict__ S, long long cap, int id, int ox0,
-                                          R acc[OXB][3][3][4]) {
-#pragma unroll
-    for (int a = 0; a < OXB; ++a)
-#pragma unroll
-        for (int oy = 0; oy < 3; ++oy)
-#pragma unroll
-            for (int oz = 0; oz < 3; ++oz) {
-                const int o = 9 * (ox0 + a) + 3 * oy + oz;
-                if (MPM_INB((long long)o * cap + id, 27 * cap, 4)) store_sum(S, (long long)o * cap + id, acc[a][oy][oz]);
-            }
-}
-
-// OXB: stencil x-offsets accumulated per pass over a cell's particles (3 or 1).
-template <typename R, int MODE, int OXB>
-__global__ void __launch_bounds__(128)
-cell_sums_kernel(Ctx ctx, const unsigned* __restrict__ perm, const R* __restrict__ payload, R* __restrict__ S,
-                 long long cap) {
-    const int nseg = *ctx.n_seg;
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nseg; id += gridDim.x * blockDim.x) {
-        const int first = ctx.seg_first[id], last = ctx.seg_last[id];
-        if (!(MPM_INB(first, ctx.n + 1, 11) && MPM_INB(last, ctx.n + 1, 11))) continue;
-#pragma unroll 1
-        for (int ox0 = 0; ox0 < 3; ox0 += OXB) {
-            R acc[OXB][3][3][4];
-            zero_acc<R, OXB>(acc);
-            for (int q = first; q < last; ++q) {
-                R r[PAYLOAD];
-                if (!MPM_INB(perm[q], ctx.n, 9)) continue;
-                load_record(payload, perm[q], r);
-                accumulate_record<R, MODE, OXB>(r, ox0, acc);
-            }
-            store_acc<R, OXB>(S, cap, id, ox0, acc);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Reverse P2G, phase 1 (transfer.py:99-119 scatter of gv_b): per occupied cell
-// the 27 stencil sums of w (nv_b + k4 Cn_b' dp), with nv_b = vn_b + dt xn_b
-// (advect) and Cn_b' = Cn_b + dt Fn_b F^T formed here from the cotangents of
-// the step's output, so no payload record is written for the reverse.
-// ---------------------------------------------------------------------------
-// the x-offsets ox_lo .. ox_lo + 3 - 1 of one occupied cell (OXB at a time)
-template <typename R, int OXB>
-__device__ __forceinline__ void adj_cell(const Ctx& ctx, const unsigned* __restrict__ perm, const MpmParticles& in,
-                                         const MpmCotangents& ob, R* __restrict__ S, long long cap, int advect,
-                                         int id, int ox_lo, int ox_hi) {
-    const int first = ctx.seg_first[id], last = ctx.seg_last[id];
-    if (!(MPM_INB(first, ctx.n, 11) && MPM_INB(last, ctx.n + 1, 11))) return;
-    const MpmScene& sc = ctx.scenes[ctx.scene_of[first]];
-    const R dx = (R)sc.dx, dt = (R)sc.dt, inv_dx = (R)(1.0 / sc.dx);
+// The reverse record of particle p (fx, -, nv_b, k4 Cn_b' dx)
+template <typename R>
+__device__ __forceinline__ void adj_record(const Ctx& ctx, const MpmParticles& in, const MpmCotangents& ob, int advect,
+                                           int scene, long long p, R r[PAYLOAD]) {
+    const SceneK<R>& sk = static_cast<const SceneK<R>*>(ctx.sk)[scene];
+    const R dx = sk.dx, dt = sk.dt, inv_dx = sk.inv_dx;
     const R kdx = R(4) * inv_dx * inv_dx * dx;
-#pragma unroll 1
-    for (int ox0 = ox_lo; ox0 < ox_hi; ox0 += OXB) {
-        R acc[OXB][3][3][3];
+    R x[3], nv[3], F[9], Fb[9], Cb[9];
+    ld3<R>(in.x, p, in.sp3, in.sc3, x);
+    ld9<R>(in.F, p, in.sp9, in.sc9, F);
+    ld9<R>(ob.F, p, ob.sp9, ob.sc9, Fb);
+    ld9<R>(ob.C, p, ob.sp9, ob.sc9, Cb);
+    ld3<R>(ob.v, p, ob.sp3, ob.sc3, nv);
+    if (advect) {
+        R xb[3];
+        ld3<R>(ob.x, p, ob.sp3, ob.sc3, xb);
 #pragma unroll
-        for (int a = 0; a < OXB; ++a)
+        for (int i = 0; i < 3; ++i) nv[i] += dt * xb[i];
+    }
+    R FbFt[9];
+    mmT(Fb, F, FbFt);
+    int base[3];
+    R fx[3];
+    bin_particle(x, inv_dx, sk.shape, base, fx);
+    r[0] = fx[0]; r[1] = fx[1]; r[2] = fx[2]; r[3] = R(0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) r[4 + i] = nv[i];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) r[7 + i] = kdx * (Cb[i] + dt * FbFt[i]);
+}
+
+// Adds one record's contributions at the stencil x-offset ox: w(o) (a + B dp(o))
+// and (forward) w(o) m in channel 0, dp = o - fx in cell units.
+template <typename R, bool ADJ>
+__device__ __forceinline__ void accumulate_record(const R r[PAYLOAD], int ox, R acc[3][3][ADJ ? 3 : 4]) {
+    R wy[3], wz[3], wx;
+    {
+        const R a = R(1.5) - r[1], b = r[1] - R(1.0), c = r[1] - R(0.5);
+        wy[0] = R(0.5) * a * a;
+        wy[1] = R(0.75) - b * b;
+        wy[2] = R(0.5) * c * c;
+    }
+    {
+        const R a = R(1.5) - r[2], b = r[2] - R(1.0), c = r[2] - R(0.5);
+        wz[0] = R(0.5) * a * a;
+        wz[1] = R(0.75) - b * b;
+        wz[2] = R(0.5) * c * c;
+    }
+    {
+        const R a = (ox == 0 ? R(1.5) : R(0.5)) - r[0], b = r[0] - R(1.0);     // (c)^2 = (-c)^2
+        wx = ox == 1 ? R(0.75) - b * b : R(0.5) * a * a;
+    }
+    const R dz[3] = {R(0) - r[2], R(1) - r[2], R(2) - r[2]};
+    const R dy[3] = {R(0) - r[1], R(1) - r[1], R(2) - r[1]};
+    const R dpx = R(ox) - r[0];
+    // a + B dp with dp = (dpx, dy, dz), x part hoisted
+    const R ax0 = r[4] + r[7] * dpx, ax1 = r[5] + r[10] * dpx, ax2 = r[6] + r[13] * dpx;
+    constexpr int M = ADJ ? 0 : 1;
+#pragma unroll
+    for (int oy = 0; oy < 3; ++oy) {
+        const R wxy = wx * wy[oy];
+        const R ay0 = ax0 + r[8] * dy[oy], ay1 = ax1 + r[11] * dy[oy], ay2 = ax2 + r[14] * dy[oy];
+#pragma unroll
+        for (int oz = 0; oz < 3; ++oz) {
+            const R wt = wxy * wz[oz];
+            if constexpr (!ADJ) acc[oy][oz][0] += wt * r[3];
+            acc[oy][oz][M + 0] += wt * (ay0 + r[9] * dz[oz]);
+            acc[oy][oz][M + 1] += wt * (ay1 + r[12] * dz[oz]);
+            acc[oy][oz][M + 2] += wt * (ay2 + r[15] * dz[oz]);
+        }
+    }
+}
+
+template <typename R, bool ADJ>
+__global__ void __launch_bounds__(32 * CellSums<R>::WARPS, CellSums<R>::MIN_CTAS)
+cell_sums_kernel(Ctx ctx, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm,
+                 const R* __restrict__ payload, MpmParticles in, MpmCotangents ob, R* __restrict__ S, int advect) {
+    constexpr int W = CellSums<R>::WARPS, CH = ADJ ? 3 : 4;
+    __shared__ __align__(16) R rec_s[W][rec_at<R>(CS_SLOTS)];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    R* rec = rec_s[warp];
+    const int c = lane / 3, ox = lane % 3;
+    const int nseg = *ctx.n_seg;
+    for (int g = (blockIdx.x * W + warp) * CS_CELLS; g < nseg; g += gridDim.x * W * CS_CELLS) {
+        const int id = g + c;
+        const int cells = nseg - g < CS_CELLS ? nseg - g : CS_CELLS;
+        const bool mine = c < cells;
+        int cur = mine ? ctx.seg_first[id] : 0;
+        int last = mine ? ctx.seg_last[id] : 0;
+        if (!(MPM_INB(cur, ctx.n + 1, 11) && MPM_INB(last, ctx.n + 1, 11))) cur = last = 0;
+        if constexpr (ADJ) {
+            if (mine && ox == 0 && cur < last) {
+                const unsigned key = skeys[cur];
+                if (MPM_INB(key, ctx.n_keys, 2)) ctx.cell_seg[key] = id + 1;
+            }
+        }
+        R acc[3][3][CH];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b)
 #pragma unroll
-                for (int c = 0; c < 3; ++c)
+                for (int h = 0; h < CH; ++h) acc[a][b][h] = R(0);
+        const int end = __reduce_max_sync(0xffffffffu, last);
+        for (;;) {
+            // the next window starts at the first slot still to be added (slots
+            // between the cells hold particles outside the grid)
+            const int w0 = __reduce_min_sync(0xffffffffu, cur < last ? cur : INT_MAX);
+            if (w0 == INT_MAX) break;
+            unsigned p[CS_SLOTS / 32];
 #pragma unroll
-                    for (int h = 0; h < 3; ++h) acc[a][b][c][h] = R(0);
-        for (int q = first; q < last; ++q) {
-            const long long p = perm[q];
-            if (!MPM_INB(p, ctx.n, 9)) continue;
-            R x[3], nv[3], B[9];
-            ld3<R>(in.x, p, in.sp3, in.sc3, x);
-            {
-                R F[9], Fb[9], Cb[9], xb[3];
-                ld9<R>(in.F, p, in.sp9, in.sc9, F);
-                ld9<R>(ob.F, p, ob.sp9, ob.sc9, Fb);
-                ld9<R>(ob.C, p, ob.sp9, ob.sc9, Cb);
-                ld3<R>(ob.v, p, ob.sp3, ob.sc3, nv);
-                if (advect) {
-                    ld3<R>(ob.x, p, ob.sp3, ob.sc3, xb);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) nv[i] += dt * xb[i];
-                }
-                R FbFt[9];
-                mmT(Fb, F, FbFt);
-#pragma unroll
-                for (int i = 0; i < 9; ++i) B[i] = kdx * (Cb[i] + dt * FbFt[i]);
+            for (int k = 0; k < CS_SLOTS / 32; ++k) {
+                const int s = w0 + 32 * k + lane;
+                p[k] = s < end ? perm[s] : 0xffffffffu;
             }
-            int base[3];
-            R fx[3];
-            bin_particle(x, inv_dx, sc.shape, base, fx);
-            R w[3][3];
-            bspline(fx, w);
-            const R dz[3] = {R(0) - fx[2], R(1) - fx[2], R(2) - fx[2]};
-            const R dy[3] = {R(0) - fx[1], R(1) - fx[1], R(2) - fx[1]};
 #pragma unroll
-            for (int a = 0; a < OXB; ++a) {
-                const int ox = ox0 + a;
-                const R dpx = R(ox) - fx[0];
-                R wx;
-                if constexpr (OXB == 3) wx = w[a][0];
-                else wx = ox == 0 ? w[0][0] : (ox == 1 ? w[1][0] : w[2][0]);
-                const R ax0 = nv[0] + B[0] * dpx, ax1 = nv[1] + B[3] * dpx, ax2 = nv[2] + B[6] * dpx;
+            for (int k = 0; k < CS_SLOTS / 32; ++k) {
+                const int s = w0 + 32 * k + lane;
+                if (s < end) {
+                    R r[PAYLOAD];
+                    if (!MPM_INB(p[k], ctx.n, 9)) {
 #pragma unroll
-                for (int oy = 0; oy < 3; ++oy) {
-                    const R wxy = wx * w[oy][1];
-                    const R ay0 = ax0 + B[1] * dy[oy], ay1 = ax1 + B[4] * dy[oy], ay2 = ax2 + B[7] * dy[oy];
-#pragma unroll
-                    for (int oz = 0; oz < 3; ++oz) {
-                        const R wt = wxy * w[oz][2];
-                        acc[a][oy][oz][0] += wt * (ay0 + B[2] * dz[oz]);
-                        acc[a][oy][oz][1] += wt * (ay1 + B[5] * dz[oz]);
-                        acc[a][oy][oz][2] += wt * (ay2 + B[8] * dz[oz]);
+                        for (int i = 0; i < PAYLOAD; ++i) r[i] = R(0);
+                    } else if constexpr (ADJ) {
+                        adj_record<R>(ctx, in, ob, advect, ctx.scene_of[s], p[k], r);
+                    } else {
+                        load_record(payload, p[k], r);
                     }
+                    put_record(rec + rec_at<R>(32 * k + lane), r);
                 }
             }
+            __syncwarp();
+            const int stop = last < w0 + CS_SLOTS ? last : w0 + CS_SLOTS;
+            for (; cur < stop; ++cur) {
+                R r[PAYLOAD];
+                get_record(rec + rec_at<R>(cur - w0), r);
+                accumulate_record<R, ADJ>(r, ox, acc);
+            }
+            __syncwarp();
         }
-#pragma unroll
-        for (int a = 0; a < OXB; ++a)
+        if (mine) {
 #pragma unroll
             for (int oy = 0; oy < 3; ++oy)
 #pragma unroll
                 for (int oz = 0; oz < 3; ++oz) {
-                    const int o = 9 * (ox0 + a) + 3 * oy + oz;
-                    const R v4[4] = {acc[a][oy][oz][0], acc[a][oy][oz][1], acc[a][oy][oz][2], R(0)};
-                    if (MPM_INB((long long)o * cap + id, 27 * cap, 4)) store_sum(S, (long long)o * cap + id, v4);
+                    const long long at = sum_at(9 * ox + 3 * oy + oz, id);
+                    R v[4];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) v[h] = h < CH ? acc[oy][oz][h] : R(0);
+                    if (MPM_INB(at, sum_entries(ctx.n), 4)) store_sum(S, at, v);
                 }
+        }
     }
-}
-
-// OXB: stencil x-offsets per pass over a cell's particles (3 or 1).
-template <typename R, int OXB>
-__global__ void __launch_bounds__(128, 4)
-cell_sums_adj_kernel(Ctx ctx, const unsigned* __restrict__ perm, MpmParticles in, MpmCotangents ob,
-                     R* __restrict__ S, long long cap, int advect) {
-    const int nseg = *ctx.n_seg;
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nseg; id += gridDim.x * blockDim.x)
-        adj_cell<R, OXB>(ctx, perm, in, ob, S, cap, advect, id, 0, 3);
 }
 
 // ---------------------------------------------------------------------------
@@ -733,7 +742,8 @@ cell_sums_adj_kernel(Ctx ctx, const unsigned* __restrict__ perm, MpmParticles in
 // active node tiles (persistent grid over the active list); every node adds
 // the sums of its 27 source cells in the fixed order o = 0..26, then
 // MODE 0: grid update -> (m, v[3]) with v = s mom/m + s dt g on free nodes;
-// MODE 1: grid adjoint -> (gm_b, gmom_b[3]) from gv_b and the forward record.
+// MODE 1: grid adjoint -> (gm_b, gmom_b[3]) from gv_b and the forward record,
+// which is also restored into the dense scratch for the reverse particle kernel.
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ __forceinline__ void load_sum(const R* __restrict__ S, long long idx, R o[4]) {
@@ -747,173 +757,95 @@ __device__ __forceinline__ void load_sum(const R* __restrict__ S, long long idx,
     }
 }
 
-// Grid adjoint of one node (the reverse node gather's epilogue): gmom_b and
-// gm_b from the gathered gv_b sums acc and the forward record, which is also
-// restored into the dense scratch for the reverse particle kernel.
-template <typename R>
-__device__ __forceinline__ void node_adjoint(const Ctx& ctx, const MpmScene& sc, const SceneAux& ax, int i, int j,
-                                             int k, long long gidx, const R acc[4], const R* __restrict__ grid_fwd,
-                                             int advect) {
-    const R s_damp = (R)(1.0 - sc.damping);
-    const R dt = (R)sc.dt;
-    const R eps = (R)sc.mass_eps;
-    const R g0 = (R)sc.gravity[0], g1 = (R)sc.gravity[1], g2 = (R)sc.gravity[2];
-    const long long didx = ax.node_begin + ((long long)i * sc.shape[1] + j) * sc.shape[2] + k;
-    if (!(MPM_INB(didx, ctx.n_nodes, 7) && MPM_INB(gidx, ctx.grid_nodes, 8))) return;
-    R rec[4] = {R(0), R(0), R(0), R(0)};
-    R f[4];
-    load_node(grid_fwd, gidx, f);
-    store_node(static_cast<R*>(ctx.dense_f), didx, f);
-    const R m = f[0];
-    if (m > eps && node_free(sc, i, j, k)) {
-        rec[1] = (s_damp * acc[0]) / m;
-        rec[2] = (s_damp * acc[1]) / m;
-        rec[3] = (s_damp * acc[2]) / m;
-        if (advect) {
-            const R sd = s_damp * dt;
-            rec[0] = -(acc[0] * (f[1] - sd * g0) + acc[1] * (f[2] - sd * g1) + acc[2] * (f[3] - sd * g2)) / m;
-        }
-    }
-    store_node(static_cast<R*>(ctx.dense_b), didx, rec);
-}
-
-// tile t of a scene -> its first node (L0, L1, L2)
-__device__ __forceinline__ void tile_origin(const SceneAux& ax, long long lt, int T, int TZ, int L[3]) {
-    const int tz = (int)(lt % ax.ntile[2]);
-    const int ty = (int)((lt / ax.ntile[2]) % ax.ntile[1]);
-    const int tx = (int)(lt / ((long long)ax.ntile[2] * ax.ntile[1]));
-    L[0] = tx * T;
-    L[1] = ty * T;
-    L[2] = tz * TZ;
-}
-
+// What bounds it: the latency of scattered loads (a node's 27 sums are 27 short
+// runs shared with its z-neighbours), so the loads are issued in groups: IDS
+// source cells' segment ids, then their sums SUMS at a time, in 64 (FP64: 80)
+// registers.  Left to the compiler's schedule the same loop took 95 to 185 us
+// on 4.7M particles, depending on the registers it settled for; in this form
+// 105 us forward and 116 us reverse, and on 4096 particles 6.5 us against 7.5
+// with 1024-thread blocks, which put a small scene on a handful of SMs.
+constexpr int NODE_THREADS = 128;
+template <typename R> struct NodeSums;
+template <> struct NodeSums<float>  { static constexpr int IDS = 9, SUMS = 9, MIN_CTAS = 8; };
+template <> struct NodeSums<double> { static constexpr int IDS = 27, SUMS = 3, MIN_CTAS = 6; };
 template <typename R, int T, int TZ, int MODE>
-__global__ void __launch_bounds__(1024)
-node_sums_kernel(Ctx ctx, const R* __restrict__ S, long long cap, const int* __restrict__ active,
+__global__ void __launch_bounds__(NODE_THREADS, NodeSums<R>::MIN_CTAS)
+node_sums_kernel(Ctx ctx, const R* __restrict__ S, const int* __restrict__ active,
                  const int* __restrict__ n_active, R* __restrict__ grid_out, const R* __restrict__ grid_fwd,
                  int advect) {
-    // Both modes walk the nodes in CTA-uniform rounds of blockDim nodes (the
-    // per-thread grid-stride form measured slower: forward 62.3 vs 65.8 ms,
-    // reverse 80.8 vs 86.7 ms per config-4 trajectory); the forward keeps its
-    // epilogue inline and the reverse calls node_adjoint, each the faster of
-    // the two measured for its mode.  The sums and their order are the same.
-    if constexpr (MODE == 0) {
-        constexpr int TN = T * T * TZ;
-        // one thread per node of the active tiles (tile-major, z fastest), grid-strided
-        const long long total = (long long)(*n_active) * TN;
-        for (long long r0 = (long long)blockIdx.x * blockDim.x; r0 < total; r0 += (long long)gridDim.x * blockDim.x) {
-            const long long gidx = r0 + threadIdx.x;
-            if (gidx >= total) continue;
-            const int it = (int)(gidx / TN), node = (int)(gidx % TN);
-            const int tile = active[it];
-            const int s = ctx.tile_scene[tile];
-            const MpmScene& sc = ctx.scenes[s];
-            const SceneAux& ax = ctx.aux[s];
-            long long lt = tile - ax.tile_begin;
-            const int tz = (int)(lt % ax.ntile[2]);
-            const int ty = (int)((lt / ax.ntile[2]) % ax.ntile[1]);
-            const int tx = (int)(lt / ((long long)ax.ntile[2] * ax.ntile[1]));
-            const int L0 = tx * T, L1 = ty * T, L2 = tz * TZ;
-            const long long P1 = sc.shape[1] + 2, P2 = sc.shape[2] + 2;
-            const R s_damp = (R)(1.0 - sc.damping);
-            const R dt = (R)sc.dt;
-            const R eps = (R)sc.mass_eps;
-            const R g0 = (R)sc.gravity[0], g1 = (R)sc.gravity[1], g2 = (R)sc.gravity[2];
-            {
-                const int nz = node % TZ, ny = (node / TZ) % T, nx = node / (TZ * T);
-                const int i = L0 + nx, j = L1 + ny, k = L2 + nz;
-                if (i >= sc.shape[0] || j >= sc.shape[1] || k >= sc.shape[2]) continue;
-                R acc[4] = {R(0), R(0), R(0), R(0)};
-                const long long cbase = ax.cell_begin + ((long long)(i + 2) * P1 + (j + 2)) * P2 + (k + 2);
-    #pragma unroll
-                for (int ox = 0; ox < 3; ++ox)
-    #pragma unroll
-                    for (int oy = 0; oy < 3; ++oy)
-    #pragma unroll
-                        for (int oz = 0; oz < 3; ++oz) {
-                            const long long ci = cbase - ((long long)ox * P1 + oy) * P2 - oz;
-                            const int id1 = MPM_INB(ci, ctx.n_keys, 6) ? ctx.cell_seg[ci] : 0;
-                            const long long si = (long long)(9 * ox + 3 * oy + oz) * cap + (id1 - 1);
-                            if (id1 && MPM_INB(si, 27 * cap, 5)) {
-                                R v[4];
-                                load_sum(S, si, v);
-                                acc[0] += v[0]; acc[1] += v[1]; acc[2] += v[2]; acc[3] += v[3];
-                            }
-                        }
-                const long long didx = ax.node_begin + ((long long)i * sc.shape[1] + j) * sc.shape[2] + k;
-                if (!(MPM_INB(didx, ctx.n_nodes, 7) && MPM_INB(gidx, ctx.grid_nodes, 8))) continue;
-                R rec[4] = {R(0), R(0), R(0), R(0)};
-                if constexpr (MODE == 0) {
-                    const R m = acc[0];
-                    rec[0] = m;
-                    if (m > eps && node_free(sc, i, j, k)) {
-                        rec[1] = (s_damp * acc[1]) / m + s_damp * dt * g0;
-                        rec[2] = (s_damp * acc[2]) / m + s_damp * dt * g1;
-                        rec[3] = (s_damp * acc[3]) / m + s_damp * dt * g2;
-                    }
-                } else {
-                    R f[4];
-                    load_node(grid_fwd, gidx, f);
-                    store_node(static_cast<R*>(ctx.dense_f), didx, f);
-                    const R m = f[0];
-                    if (m > eps && node_free(sc, i, j, k)) {
-                        rec[1] = (s_damp * acc[0]) / m;
-                        rec[2] = (s_damp * acc[1]) / m;
-                        rec[3] = (s_damp * acc[2]) / m;
-                        if (advect) {
-                            const R sd = s_damp * dt;
-                            rec[0] = -(acc[0] * (f[1] - sd * g0) + acc[1] * (f[2] - sd * g1) + acc[2] * (f[3] - sd * g2)) / m;
-                        }
-                    }
+    constexpr unsigned TN = T * T * TZ;
+    constexpr int IDS = NodeSums<R>::IDS, G = NodeSums<R>::SUMS;
+    // one thread per node of the active tiles (tile-major, z fastest), grid-strided
+    const long long total = (long long)(*n_active) * TN;
+    for (long long gidx = (long long)blockIdx.x * NODE_THREADS + threadIdx.x; gidx < total;
+         gidx += (long long)gridDim.x * NODE_THREADS) {
+        const int tile = active[gidx / TN];
+        const unsigned node = (unsigned)(gidx % TN);
+        const int s = ctx.tile_scene[tile];
+        const SceneK<R>& sc = static_cast<const SceneK<R>*>(ctx.sk)[s];
+        const SceneAux& ax = ctx.aux[s];
+        // the scene's tiles and nodes fit 32 bits (its padded cells do)
+        const unsigned lt = (unsigned)(tile - ax.tile_begin), nt1 = ax.ntile[1], nt2 = ax.ntile[2];
+        const unsigned row = lt / nt2, tx = row / nt1;
+        const int i = (int)(tx * T + node / (TZ * T)), j = (int)((row - tx * nt1) * T + (node / TZ) % T),
+                  k = (int)((lt - row * nt2) * TZ + node % TZ);
+        if (i >= sc.shape[0] || j >= sc.shape[1] || k >= sc.shape[2]) continue;
+        const int P1 = sc.shape[1] + 2, P2 = sc.shape[2] + 2;
+        const long long cbase = ax.cell_begin + (((i + 2) * P1 + (j + 2)) * P2 + (k + 2));
+        R f[4];
+        if (MODE == 1 && MPM_INB(gidx, ctx.grid_nodes, 8)) load_node(grid_fwd, gidx, f);
+        R acc[4] = {R(0), R(0), R(0), R(0)};
+#pragma unroll
+        for (int o0 = 0; o0 < 27; o0 += IDS) {
+            int id[IDS];
+#pragma unroll
+            for (int g = 0; g < IDS; ++g) {
+                const int o = o0 + g;
+                const long long ci = cbase - ((o / 9) * P1 + (o / 3) % 3) * P2 - o % 3;
+                id[g] = MPM_INB(ci, ctx.n_keys, 6) ? ctx.cell_seg[ci] : 0;
+            }
+#pragma unroll
+            for (int g0 = 0; g0 < IDS; g0 += G) {
+                R v[G][4];
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const long long si = sum_at(o0 + g0 + g, id[g0 + g] - 1);
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) v[g][h] = R(0);
+                    if (id[g0 + g] != 0 && MPM_INB(si, sum_entries(ctx.n), 5)) load_sum(S, si, v[g]);
                 }
-                if constexpr (MODE == 0) {
-                    store_node(grid_out, gidx, rec);
-                    store_node(static_cast<R*>(ctx.dense_f), didx, rec);
-                } else {
-                    store_node(static_cast<R*>(ctx.dense_b), didx, rec);
-                }
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+#pragma unroll
+                    for (int h = 0; h < (MODE == 0 ? 4 : 3); ++h) acc[h] += v[g][h];
             }
         }
-    } else {
-        constexpr int TN = T * T * TZ;
-        // one thread per node of the active tiles (tile-major, z fastest), grid-strided
-        const int nact = *n_active;
-        const long long total = (long long)nact * TN;
-        const long long stride = (long long)gridDim.x * blockDim.x;
-        // (a CTA-uniform loop over rounds of blockDim nodes: 80.8 ms per config-4
-        // trajectory against 86.7 for the per-thread grid-stride form)
-        for (long long r0 = (long long)blockIdx.x * blockDim.x; r0 < total; r0 += stride) {
-            const long long gidx = r0 + threadIdx.x;
-            if (gidx >= total) continue;
-            const int it = (int)(gidx / TN), node = (int)(gidx % TN);
-            const int tile = active[it];
-            const int s = ctx.tile_scene[tile];
-            const MpmScene& sc = ctx.scenes[s];
-            const SceneAux& ax = ctx.aux[s];
-            int L[3];
-            tile_origin(ax, tile - ax.tile_begin, T, TZ, L);
-            const long long P1 = sc.shape[1] + 2, P2 = sc.shape[2] + 2;
-            const int nz = node % TZ, ny = (node / TZ) % T, nx = node / (TZ * T);
-            const int i = L[0] + nx, j = L[1] + ny, k = L[2] + nz;
-            if (i >= sc.shape[0] || j >= sc.shape[1] || k >= sc.shape[2]) continue;
-            R acc[4] = {R(0), R(0), R(0), R(0)};
-            const long long cbase = ax.cell_begin + ((long long)(i + 2) * P1 + (j + 2)) * P2 + (k + 2);
+        const long long didx = ax.node_begin + ((i * sc.shape[1] + j) * sc.shape[2] + k);
+        if (!(MPM_INB(didx, ctx.n_nodes, 7) && MPM_INB(gidx, ctx.grid_nodes, 8))) continue;
+        const R s_damp = sc.s_damp, dt = sc.dt;
+        R rec[4] = {R(0), R(0), R(0), R(0)};
+        if constexpr (MODE == 0) {
+            const R m = acc[0];
+            rec[0] = m;
+            if (m > sc.mass_eps && node_free(sc, i, j, k)) {
 #pragma unroll
-            for (int ox = 0; ox < 3; ++ox)
+                for (int d = 0; d < 3; ++d) rec[1 + d] = (s_damp * acc[1 + d]) / m + s_damp * dt * sc.gravity[d];
+            }
+            store_node(grid_out, gidx, rec);
+            store_node(static_cast<R*>(ctx.dense_f), didx, rec);
+        } else {
+            store_node(static_cast<R*>(ctx.dense_f), didx, f);
+            const R m = f[0];
+            if (m > sc.mass_eps && node_free(sc, i, j, k)) {
 #pragma unroll
-                for (int oy = 0; oy < 3; ++oy)
-#pragma unroll
-                    for (int oz = 0; oz < 3; ++oz) {
-                        const long long ci = cbase - ((long long)ox * P1 + oy) * P2 - oz;
-                        const int id1 = MPM_INB(ci, ctx.n_keys, 6) ? ctx.cell_seg[ci] : 0;
-                        const long long si = (long long)(9 * ox + 3 * oy + oz) * cap + (id1 - 1);
-                        if (id1 && MPM_INB(si, 27 * cap, 5)) {
-                            R v[4];
-                            load_sum(S, si, v);
-                            acc[0] += v[0]; acc[1] += v[1]; acc[2] += v[2]; acc[3] += v[3];
-                        }
-                    }
-            node_adjoint<R>(ctx, sc, ax, i, j, k, gidx, acc, grid_fwd, advect);
+                for (int d = 0; d < 3; ++d) rec[1 + d] = (s_damp * acc[d]) / m;
+                if (advect) {
+                    const R sd = s_damp * dt;
+                    rec[0] = -(acc[0] * (f[1] - sd * sc.gravity[0]) + acc[1] * (f[2] - sd * sc.gravity[1])
+                             + acc[2] * (f[3] - sd * sc.gravity[2])) / m;
+                }
+            }
+            store_node(static_cast<R*>(ctx.dense_b), didx, rec);
         }
     }
 }
