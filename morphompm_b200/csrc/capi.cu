@@ -69,7 +69,8 @@ struct MpmPlan {
     std::vector<long long> run_begin, run_end;
     bool runs_grouped = false;
     long long n_nodes = 0;
-    size_t o_dbuf, o_tape;
+    size_t o_dbuf, o_part, o_arrived, o_tape;     // per-slot gradients, their chunk sums, a counter per scene
+    int reduce_chunks = 1;                        // of the largest scene
     int nblk_seg = 1, nblk_tile = 1;
     // the state whose keys and P2G records the last MPM_FWD_EMIT call formed
     bool chain_valid = false;
@@ -510,6 +511,20 @@ int step_fwd_R(MpmPlan* P, const MpmParticles& in, MpmParticles& out, int advect
     return check_launch();
 }
 
+// per-scene sums of a per-slot buffer (at most 65535 scenes per launch: grid.y)
+void launch_reduce(MpmPlan* P, const Ctx& ctx, const double* v, double* out, int accumulate, int mean, int stride,
+                   cudaStream_t st) {
+    const size_t S = P->scenes.size();
+    for (size_t s0 = 0; s0 < S; s0 += 65535) {
+        Ctx c = ctx;
+        c.scenes += s0;
+        const unsigned ns = (unsigned)std::min<size_t>(65535, S - s0);
+        scene_reduce_kernel<<<dim3((unsigned)P->reduce_chunks, ns), REDUCE_THREADS, 0, st>>>(
+            c, v, out + s0 * stride, at<double>(P, P->o_part) + s0 * P->reduce_chunks,
+            at<unsigned>(P, P->o_arrived) + s0, accumulate, mean, stride);
+    }
+}
+
 template <typename R>
 int step_bwd_R(MpmPlan* P, const MpmParticles& in, const void* outC, const MpmCotangents& ob, MpmCotangents& ib,
                double* growth_grad, double* material_grad, int advect, int t, const char* tape, cudaStream_t st) {
@@ -557,13 +572,12 @@ int step_bwd_R(MpmPlan* P, const MpmParticles& in, const void* outC, const MpmCo
     }
     if (want_dA) {
         Site s(P, MPM_K_REDUCE, 1, st);
-        scene_reduce_kernel<<<(int)P->scenes.size(), REDUCE_THREADS, 0, st>>>(ctx, dbuf, growth_grad, 1, 0);
+        launch_reduce(P, ctx, dbuf, growth_grad, 1, 0, 1, st);
     }
     if (material_grad) {
         Site s(P, MPM_K_REDUCE, 2, st);
-        scene_reduce_kernel<<<(int)P->scenes.size(), REDUCE_THREADS, 0, st>>>(ctx, dmat, material_grad, 1, 0, 2);
-        scene_reduce_kernel<<<(int)P->scenes.size(), REDUCE_THREADS, 0, st>>>(ctx, dmat + P->n, material_grad + 1,
-                                                                             1, 0, 2);
+        launch_reduce(P, ctx, dmat, material_grad, 1, 0, 2, st);
+        launch_reduce(P, ctx, dmat + P->n, material_grad + 1, 1, 0, 2, st);
     }
     return check_launch();
 }
@@ -716,6 +730,10 @@ int mpm_plan_create(const MpmScene* scenes, int32_t n_scenes, int32_t real_bytes
     P->o_dense_f = L.take((size_t)P->n_nodes * 4 * R);
     P->o_dense_b = L.take((size_t)P->n_nodes * 4 * R);
     P->o_dbuf = L.take(3 * n * 8);      // dL/dA, dL/dmu, dL/dlambda per slot
+    for (const MpmScene& sc : P->scenes)
+        P->reduce_chunks = std::max(P->reduce_chunks, (int)((sc.p_end - sc.p_begin + REDUCE_CHUNK - 1) / REDUCE_CHUNK));
+    P->o_part = L.take((size_t)P->reduce_chunks * P->scenes.size() * 8);
+    P->o_arrived = L.take(P->scenes.size() * 4);
     const size_t nw = (n + 31) / 32;
     P->nblk_resort = (int)((nw + RESORT_THREADS - 1) / RESORT_THREADS);
     P->o_mflag = L.take(nw * 32);
@@ -824,6 +842,7 @@ int mpm_plan_bind(MpmPlan* P, void* workspace, void* stream) {
         cudaMemcpyAsync(P->ws + P->o_tile_scene, P->tile_scene.data(), 4 * P->tile_scene.size(),
                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_status, 0, 128, st) != cudaSuccess ||
+        cudaMemsetAsync(P->ws + P->o_arrived, 0, P->scenes.size() * 4, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_cell_seg, 0, (size_t)P->n_keys * 4, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_tile_flag, 0, (size_t)P->n_tiles * 4, st) != cudaSuccess)
         return MPM_ERR_CUDA;
@@ -1216,7 +1235,7 @@ int mpm_loss_detF(MpmPlan* P, const void* F, int64_t sp9, int64_t sc9, double* l
         loss_detF_kernel<float><<<g, 256, 0, st>>>(ctx, (const float*)F, sp9, sc9, dbuf, (float*)F_bar);
     else
         loss_detF_kernel<double><<<g, 256, 0, st>>>(ctx, (const double*)F, sp9, sc9, dbuf, (double*)F_bar);
-    scene_reduce_kernel<<<(int)P->scenes.size(), REDUCE_THREADS, 0, st>>>(ctx, dbuf, loss, 0, 0);
+    launch_reduce(P, ctx, dbuf, loss, 0, 0, 1, st);
     return check_launch();
 }
 
@@ -1234,7 +1253,7 @@ int mpm_loss_mse(MpmPlan* P, const void* x, int64_t sp3, int64_t sc3, const void
     else
         loss_mse_kernel<double><<<g, 256, 0, st>>>(ctx, (const double*)x, sp3, sc3, (const double*)x_obs, dbuf,
                                                    (double*)x_bar);
-    scene_reduce_kernel<<<(int)P->scenes.size(), REDUCE_THREADS, 0, st>>>(ctx, dbuf, loss, 0, 1);
+    launch_reduce(P, ctx, dbuf, loss, 0, 1, 1, st);
     return check_launch();
 }
 

@@ -1234,36 +1234,69 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
 // deterministic per-scene reduction of a per-slot double buffer:
 // out[s * stride] = (accumulate ? out[s * stride] : 0) + scale_s * sum_{slots of s} v
 // scale_s = 1 (mode 0) or 1/n_s (mode 1)
+// Block (c, s) sums chunk c of REDUCE_CHUNK slots of scene s; the last block of
+// a scene to arrive (a counter per scene, back at 0 afterwards) adds the
+// chunks' sums in chunk order, so the order depends only on the scene's size.
+// One block per scene took 242 us on a scene of 2.1M particles, on one SM; its
+// 64 chunks take 10 us.  A second block costs about 1 us of waiting, so a
+// chunk is as large as still pays: one scene of 32768 particles 4.3 us whole,
+// 5.3 in two chunks; 256 scenes of up to 65536 14.8 us, 19.1 in chunks of 8192.
 // ---------------------------------------------------------------------------
 constexpr int REDUCE_THREADS = 1024;
-__global__ void __launch_bounds__(REDUCE_THREADS)
-scene_reduce_kernel(Ctx ctx, const double* __restrict__ v, double* __restrict__ out, int accumulate, int mean,
-                    int stride = 1) {
-    __shared__ double wsum[REDUCE_THREADS / 32];
-    const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const MpmScene& sc = ctx.scenes[s];
-    // two interleaved chains per thread, then a fixed shuffle tree: the order
-    // depends only on the scene's size
-    double a0 = 0.0, a1 = 0.0;
-    long long i = sc.p_begin + threadIdx.x;
-    for (; i + REDUCE_THREADS < sc.p_end; i += 2 * REDUCE_THREADS) {
-        a0 += v[i];
-        a1 += v[i + REDUCE_THREADS];
-    }
-    if (i < sc.p_end) a0 += v[i];
-    double acc = a0 + a1;
+constexpr int REDUCE_CHUNK = 32768;
+// sum of one value per thread over the block, on thread 0 (fixed shuffle tree)
+__device__ __forceinline__ double reduce_block(double acc, double* wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0) wsum[warp] = acc;
     __syncthreads();
+    double r = 0.0;
     if (warp == 0) {
-        double r = wsum[lane];
+        r = wsum[lane];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
-        if (lane == 0) {
-            if (mean) r /= (double)(sc.p_end - sc.p_begin > 0 ? sc.p_end - sc.p_begin : 1);
-            out[(long long)s * stride] = accumulate ? out[(long long)s * stride] + r : r;
+    }
+    return r;
+}
+__global__ void __launch_bounds__(REDUCE_THREADS)
+scene_reduce_kernel(Ctx ctx, const double* __restrict__ v, double* __restrict__ out, double* __restrict__ part,
+                    unsigned* __restrict__ arrived, int accumulate, int mean, int stride = 1) {
+    __shared__ double wsum[REDUCE_THREADS / 32];
+    __shared__ bool is_last;
+    const int s = blockIdx.y, c = blockIdx.x;
+    const long long b = ctx.scenes[s].p_begin, e = ctx.scenes[s].p_end;
+    const int chunks = e > b ? (int)((e - b + REDUCE_CHUNK - 1) / REDUCE_CHUNK) : 1;
+    if (c >= chunks) return;
+    const long long c0 = b + (long long)c * REDUCE_CHUNK, c1 = c0 + REDUCE_CHUNK < e ? c0 + REDUCE_CHUNK : e;
+    // two interleaved chains per thread, then a fixed shuffle tree
+    double a0 = 0.0, a1 = 0.0;
+    long long i = c0 + threadIdx.x;
+#pragma unroll 4
+    for (; i + REDUCE_THREADS < c1; i += 2 * REDUCE_THREADS) {
+        a0 += v[i];
+        a1 += v[i + REDUCE_THREADS];
+    }
+    if (i < c1) a0 += v[i];
+    double r = reduce_block(a0 + a1, wsum);
+    if (chunks > 1) {
+        double* mine = part + (long long)s * gridDim.x;
+        if (threadIdx.x == 0) {
+            mine[c] = r;
+            __threadfence();
+            is_last = atomicAdd(arrived + s, 1u) == (unsigned)chunks - 1u;
         }
+        __syncthreads();
+        if (!is_last) return;
+        __threadfence();
+        double a = 0.0;
+        for (int k = threadIdx.x; k < chunks; k += REDUCE_THREADS) a += __ldcg(mine + k);
+        r = reduce_block(a, wsum);
+        if (threadIdx.x == 0) arrived[s] = 0u;
+    }
+    if (threadIdx.x == 0) {
+        if (mean) r /= (double)(e - b > 0 ? e - b : 1);
+        out[(long long)s * stride] = accumulate ? out[(long long)s * stride] + r : r;
     }
 }
 
