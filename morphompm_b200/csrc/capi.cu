@@ -582,6 +582,19 @@ int step_bwd_R(MpmPlan* P, const MpmParticles& in, const void* outC, const MpmCo
     return check_launch();
 }
 
+// f(real value, model constant) for a real size and a built-in model; any
+// other model value runs as neo-Hookean, as in the run-time switch
+template <typename Fn>
+int for_real_model(int real_bytes, int model, Fn&& f) {
+    auto with = [&](auto real) {
+        if (model == MPM_MODEL_HENCKY) return f(real, std::integral_constant<int, MPM_MODEL_HENCKY>{});
+        if (model == MPM_MODEL_HERSCHEL_BULKLEY)
+            return f(real, std::integral_constant<int, MPM_MODEL_HERSCHEL_BULKLEY>{});
+        return f(real, std::integral_constant<int, MPM_MODEL_NEOHOOKEAN>{});
+    };
+    return real_bytes == 4 ? with(float{}) : with(double{});
+}
+
 bool scene_ok(const MpmScene& s) {
     for (int d = 0; d < 3; ++d)
         if (s.shape[d] < 1 || s.shape[d] > 4096) return false;
@@ -1179,14 +1192,12 @@ int mpm_stress(const MpmScene* scene, int32_t real_bytes, int64_t n, const void*
     if (scene->model == MPM_MODEL_EXTERNAL) return MPM_ERR_UNSUPPORTED;
     if (n == 0) return MPM_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int g = grid_for(n, 256);
-    if (real_bytes == 4)
-        stress_kernel<float><<<g, 256, 0, st>>>(*scene, n, (const float*)F, (const float*)Fg, (const float*)C,
-                                                (float*)tau, 1e-6f);
-    else
-        stress_kernel<double><<<g, 256, 0, st>>>(*scene, n, (const double*)F, (const double*)Fg,
-                                                 (const double*)C, (double*)tau, 0.0f);
-    return check_launch();
+    return for_real_model(real_bytes, scene->model, [&](auto real, auto kind) {
+        using R = decltype(real);
+        stress_kernel<R, decltype(kind)::value><<<grid_for(n, SEAM_THREADS), SEAM_THREADS, 0, st>>>(
+            *scene, n, (const R*)F, (const R*)Fg, (const R*)C, (R*)tau, sizeof(R) == 4 ? 1e-6f : 0.0f);
+        return check_launch();
+    });
 }
 
 int mpm_stress_vjp(const MpmScene* scene, int32_t real_bytes, int64_t n, const void* F, const void* Fg,
@@ -1196,16 +1207,13 @@ int mpm_stress_vjp(const MpmScene* scene, int32_t real_bytes, int64_t n, const v
     if (scene->model == MPM_MODEL_EXTERNAL) return MPM_ERR_UNSUPPORTED;
     if (n == 0) return MPM_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int g = grid_for(n, 256);
-    if (real_bytes == 4)
-        stress_vjp_kernel<float><<<g, 256, 0, st>>>(*scene, n, (const float*)F, (const float*)Fg, (const float*)C,
-                                                    (const float*)tau_bar, (float*)F_bar, (float*)Fg_bar,
-                                                    (float*)C_bar, 1e-6f);
-    else
-        stress_vjp_kernel<double><<<g, 256, 0, st>>>(*scene, n, (const double*)F, (const double*)Fg,
-                                                     (const double*)C, (const double*)tau_bar, (double*)F_bar,
-                                                     (double*)Fg_bar, (double*)C_bar, 0.0f);
-    return check_launch();
+    return for_real_model(real_bytes, scene->model, [&](auto real, auto kind) {
+        using R = decltype(real);
+        stress_vjp_kernel<R, decltype(kind)::value><<<grid_for(n, SEAM_THREADS), SEAM_THREADS, 0, st>>>(
+            *scene, n, (const R*)F, (const R*)Fg, (const R*)C, (const R*)tau_bar, (R*)F_bar, (R*)Fg_bar, (R*)C_bar,
+            sizeof(R) == 4 ? 1e-6f : 0.0f);
+        return check_launch();
+    });
 }
 
 int mpm_bin_keys(const MpmScene* scene, int32_t real_bytes, int64_t n, const void* x, int32_t* keys, void* stream) {

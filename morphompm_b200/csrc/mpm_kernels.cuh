@@ -1345,51 +1345,90 @@ loss_mse_kernel(Ctx ctx, const R* __restrict__ x, long long sp3, long long sc3, 
 }
 
 // ---------------------------------------------------------------------------
-// constitutive seam, batched over n particles of one model
+// constitutive seam, batched over n particles of one model.  The (n, 3, 3)
+// arrays are contiguous: a warp moves the 288 values of its 32 particles as
+// nine coalesced rows through shared memory (a lane's own nine values lie 9
+// apart there, on distinct banks), so every sector is fetched once.  With the
+// strided loads and the out-of-line Hencky VJP, whose arrays went through the
+// local-memory stack, the pair took 215 us on 1.05M FP32 Hencky particles (37
+// stress, 167 VJP), now 110 (39 and 64: the eigensolve's instructions bound
+// both); neo-Hookean 199, now 80; Herschel-Bulkley 197, now 94; FP64 374, 268
+// and 274, now 250, 116 and 170.
 // ---------------------------------------------------------------------------
+constexpr int SEAM_THREADS = 128;
 template <typename R>
-__global__ void __launch_bounds__(256)
-stress_kernel(MpmScene sc, long long n, const R* __restrict__ F, const R* __restrict__ Fg, const R* __restrict__ C,
-              R* __restrict__ tau, float thresh) {
-    long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    ModelParams<R> M;
-    M.load(sc);
-    R f[9], g[9], c[9], t[9];
+__device__ __forceinline__ void seam_load(const R* __restrict__ A, long long w0, long long n, R* sh, R o[9]) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        f[i] = F[9 * p + i];
-        g[i] = Fg[9 * p + i];
-        c[i] = C ? C[9 * p + i] : R(0);
+    for (int k = 0; k < 9; ++k) {
+        const long long e = 9 * w0 + 32 * k + lane;
+        sh[32 * k + lane] = e < 9 * n ? A[e] : ((32 * k + lane) % 9 % 4 == 0 ? R(1) : R(0));
     }
-    model_stress(M, thresh, f, g, c, t);
+    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 9; ++i) tau[9 * p + i] = t[i];
+    for (int i = 0; i < 9; ++i) o[i] = sh[9 * lane + i];
 }
 template <typename R>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ void seam_store(R* __restrict__ A, long long w0, long long n, R* sh, const R o[9]) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 9; ++i) sh[9 * lane + i] = o[i];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const long long e = 9 * w0 + 32 * k + lane;
+        if (e < 9 * n) A[e] = sh[32 * k + lane];
+    }
+}
+// KIND: the scene's model.  The elastic models do not read C.
+template <typename R, int KIND>
+__global__ void __launch_bounds__(SEAM_THREADS, sizeof(R) == 4 ? 10 : 8)
+stress_kernel(MpmScene sc, long long n, const R* __restrict__ F, const R* __restrict__ Fg, const R* __restrict__ C,
+              R* __restrict__ tau, float thresh) {
+    __shared__ R sh_all[SEAM_THREADS / 32][288];
+    R* sh = sh_all[threadIdx.x >> 5];
+    const long long w0 = (long long)blockIdx.x * SEAM_THREADS + (threadIdx.x & ~31);    // the warp's first particle
+    if (w0 >= n) return;
+    ModelParams<R> M;
+    M.load(sc);
+    M.kind = KIND;
+    R f[9], g[9], c[9], t[9];
+    seam_load(F, w0, n, sh, f);
+    seam_load(Fg, w0, n, sh, g);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) c[i] = R(0);
+    if (KIND == MPM_MODEL_HERSCHEL_BULKLEY && C) seam_load(C, w0, n, sh, c);
+    model_stress(M, thresh, f, g, c, t);
+    seam_store(tau, w0, n, sh, t);
+}
+template <typename R, int KIND>
+__global__ void __launch_bounds__(SEAM_THREADS, sizeof(R) == 4 ? 7 : 5)
 stress_vjp_kernel(MpmScene sc, long long n, const R* __restrict__ F, const R* __restrict__ Fg,
                   const R* __restrict__ C, const R* __restrict__ tb, R* __restrict__ Fb, R* __restrict__ Fgb,
                   R* __restrict__ Cb, float thresh) {
-    long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
+    __shared__ R sh_all[SEAM_THREADS / 32][288];
+    R* sh = sh_all[threadIdx.x >> 5];
+    const long long w0 = (long long)blockIdx.x * SEAM_THREADS + (threadIdx.x & ~31);
+    if (w0 >= n) return;
     ModelParams<R> M;
     M.load(sc);
+    M.kind = KIND;
     R f[9], g[9], c[9], t[9], a[9], b[9], e[9];
+    seam_load(F, w0, n, sh, f);
+    seam_load(Fg, w0, n, sh, g);
+    seam_load(tb, w0, n, sh, t);
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        f[i] = F[9 * p + i];
-        g[i] = Fg[9 * p + i];
-        c[i] = C ? C[9 * p + i] : R(0);
-        t[i] = tb[9 * p + i];
-    }
-    model_vjp(M, thresh, f, g, c, t, a, b, e);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        Fb[9 * p + i] = a[i];
-        Fgb[9 * p + i] = b[i];
-        if (Cb) Cb[9 * p + i] = e[i];
-    }
+    for (int i = 0; i < 9; ++i) c[i] = e[i] = R(0);
+    if (KIND == MPM_MODEL_HERSCHEL_BULKLEY && C) seam_load(C, w0, n, sh, c);
+    if constexpr (KIND == MPM_MODEL_HENCKY)
+        Hencky<R>::vjp(f, g, M.mu, M.lam, thresh, t, a, b);
+    else
+        model_vjp(M, thresh, f, g, c, t, a, b, e);
+    seam_store(Fb, w0, n, sh, a);
+    seam_store(Fgb, w0, n, sh, b);
+    if (Cb) seam_store(Cb, w0, n, sh, e);
 }
 
 }  // namespace mpm
