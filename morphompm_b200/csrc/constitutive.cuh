@@ -186,7 +186,8 @@ struct ModelParams {
     int kind;
     R mu, lam;
     R kappa, K, n, tau_y, m, eps;
-    __device__ __forceinline__ void load(const MpmScene& sc) {
+    template <typename Scene>       // MpmScene or SceneK<R>
+    __device__ __forceinline__ void load(const Scene& sc) {
         kind = sc.model;
         mu = (R)sc.mu; lam = (R)sc.lam;
         kappa = (R)sc.kappa; K = (R)sc.K; n = (R)sc.n_exp;
@@ -194,25 +195,81 @@ struct ModelParams {
     }
 };
 
-// F_bar = Fe_bar Fg^{-T};  Fg_bar = -Fg^{-T} F^T Fe_bar Fg^{-T}   (constitutive.py:37-38, 73-74)
+// Growth tensor of a particle.  GrowthFull: any Fg, 9 values of the caller's.
+// GrowthIso: Fg = g I, with the values that the 3x3 formulas give for it (its
+// zeros cannot be folded away there: 0 * x is not 0 for every x).  It spares
+// the reverse particle kernel about 250 instructions and G2P about 60.
 template <typename R>
-__device__ __forceinline__ void pull_back(const R F[9], const R Fgi[9], const R Feb[9], R Fb[9], R Fgb[9]) {
-    mmT(Feb, Fgi, Fb);              // Fe_bar Fg^{-T}
-    R T1[9], T2[9];
-    mTm(F, Fb, T1);                 // F^T (Fe_bar Fg^{-T})
-    mTm(Fgi, T1, T2);               // Fg^{-T} F^T Fe_bar Fg^{-T}
+struct GrowthFull {
+    static constexpr bool ISO = false;
+    R Fg[9];
+    GrowthFull() = default;
+    __device__ __forceinline__ explicit GrowthFull(const R* v) {
 #pragma unroll
-    for (int i = 0; i < 9; ++i) Fgb[i] = -T2[i];
-}
+        for (int i = 0; i < 9; ++i) Fg[i] = v[i];
+    }
+    __device__ __forceinline__ R det() const { return det3(Fg); }
+    __device__ __forceinline__ R inverse(R Fgi[9]) const { return inv3(Fg, Fgi); }
+    __device__ __forceinline__ void full(R o[9]) const {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) o[i] = Fg[i];
+    }
+    // Fe = F Fg^{-1}
+    __device__ __forceinline__ void elastic(const R F[9], R Fe[9]) const {
+        R Fgi[9];
+        inv3(Fg, Fgi);
+        mm(F, Fgi, Fe);
+    }
+    // F_bar = Fe_bar Fg^{-T};  Fg_bar = -Fg^{-T} F^T Fe_bar Fg^{-T}   (constitutive.py:37-38, 73-74)
+    __device__ __forceinline__ void pull_back(const R F[9], const R Feb[9], R Fb[9], R Fgb[9]) const {
+        R Fgi[9], T1[9], T2[9];
+        inv3(Fg, Fgi);
+        mmT(Feb, Fgi, Fb);              // Fe_bar Fg^{-T}
+        mTm(F, Fb, T1);                 // F^T (Fe_bar Fg^{-T})
+        mTm(Fgi, T1, T2);               // Fg^{-T} F^T Fe_bar Fg^{-T}
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Fgb[i] = -T2[i];
+    }
+};
+template <typename R>
+struct GrowthIso {
+    static constexpr bool ISO = true;
+    R g;
+    __device__ __forceinline__ R det() const { return g * (g * g); }
+    __device__ __forceinline__ R inv() const { return (g * g) * (R(1) / (g * (g * g))); }
+    __device__ __forceinline__ R inverse(R Fgi[9]) const {
+        const R v = inv();
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Fgi[i] = (i % 4 == 0) ? v : R(0);
+        return det();
+    }
+    __device__ __forceinline__ void full(R o[9]) const {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) o[i] = (i % 4 == 0) ? g : R(0);
+    }
+    __device__ __forceinline__ void elastic(const R F[9], R Fe[9]) const {
+        const R v = inv();
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Fe[i] = F[i] * v;
+    }
+    __device__ __forceinline__ void pull_back(const R F[9], const R Feb[9], R Fb[9], R Fgb[9]) const {
+        const R v = inv();
+        R T1[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Fb[i] = Feb[i] * v;
+        mTm(F, Fb, T1);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Fgb[i] = -(v * T1[i]);
+    }
+};
 
 // ---------------------------------------------------------------------------
 // neo-Hookean: tau = mu (Fe Fe^T - I) + lam ln J I
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ void nh_stress(const R F[9], const R Fg[9], R mu, R lam, R tau[9]) {
-    R Fgi[9], Fe[9];
-    inv3(Fg, Fgi);
-    mm(F, Fgi, Fe);
+template <typename R, typename G>
+__device__ __forceinline__ void nh_stress(const R F[9], const G& g, R mu, R lam, R tau[9]) {
+    R Fe[9];
+    g.elastic(F, Fe);
     R J = det3(Fe);
     R lnJ = d_log(J);
     mmT(Fe, Fe, tau);
@@ -220,12 +277,11 @@ __device__ __forceinline__ void nh_stress(const R F[9], const R Fg[9], R mu, R l
     for (int i = 0; i < 9; ++i) tau[i] = mu * (tau[i] - ((i % 4 == 0) ? R(1) : R(0)));
     tau[0] += lam * lnJ; tau[4] += lam * lnJ; tau[8] += lam * lnJ;
 }
-template <typename R>
-__device__ __forceinline__ void nh_vjp(const R F[9], const R Fg[9], R mu, R lam, const R tau_bar[9],
+template <typename R, typename G>
+__device__ __forceinline__ void nh_vjp(const R F[9], const G& g, R mu, R lam, const R tau_bar[9],
                                        R Fb[9], R Fgb[9]) {
-    R Fgi[9], Fe[9], Fei[9], tb[9];
-    inv3(Fg, Fgi);
-    mm(F, Fgi, Fe);
+    R Fe[9], Fei[9], tb[9];
+    g.elastic(F, Fe);
     inv3(Fe, Fei);
     sym(tau_bar, tb);
     R tr = tb[0] + tb[4] + tb[8];
@@ -236,7 +292,7 @@ __device__ __forceinline__ void nh_vjp(const R F[9], const R Fg[9], R mu, R lam,
 #pragma unroll
         for (int j = 0; j < 3; ++j)
             Feb[3 * i + j] = R(2) * mu * T[3 * i + j] + lam * tr * Fei[3 * j + i];
-    pull_back(F, Fgi, Feb, Fb, Fgb);
+    g.pull_back(F, Feb, Fb, Fgb);
 }
 
 // ---------------------------------------------------------------------------
@@ -247,10 +303,9 @@ __device__ __forceinline__ void nh_vjp(const R F[9], const R Fg[9], R mu, R lam,
 // recomputes particles whose relative singular-value gap is below the
 // threshold in FP64.
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ void hencky_eig(const R F[9], const R Fg[9], R Fgi[9], R Fe[9], R beta[3], R V[9]) {
-    inv3(Fg, Fgi);
-    mm(F, Fgi, Fe);
+template <typename R, typename G>
+__device__ __forceinline__ void hencky_eig(const R F[9], const G& g, R Fe[9], R beta[3], R V[9]) {
+    g.elastic(F, Fe);
     R b[9];
     mmT(Fe, Fe, b);
     if constexpr (sizeof(R) == 4) {
@@ -300,8 +355,8 @@ __device__ __forceinline__ double dk_stable(double bi, double bj) {
 }
 
 // STABLE: the cancellation-free divided difference also in FP64.
-template <typename R, bool STABLE = false>
-__device__ __forceinline__ void hencky_vjp_from_eig(const R F[9], const R Fgi[9], const R Fe[9], const R beta[3],
+template <bool STABLE, typename R, typename G>
+__device__ __forceinline__ void hencky_vjp_from_eig(const R F[9], const G& g, const R Fe[9], const R beta[3],
                                                     const R V[9], R mu, R lam, const R tau_bar[9],
                                                     R Fb[9], R Fgb[9]) {
     R tb[9];
@@ -352,7 +407,7 @@ __device__ __forceinline__ void hencky_vjp_from_eig(const R F[9], const R Fgi[9]
     mm(Bb, Fe, Feb);
 #pragma unroll
     for (int i = 0; i < 9; ++i) Feb[i] *= R(2);
-    pull_back(F, Fgi, Feb, Fb, Fgb);
+    g.pull_back(F, Feb, Fb, Fgb);
 }
 
 // relative singular-value gap: min |s_i - s_j| / max s  with s = sqrt(beta)
@@ -372,17 +427,19 @@ __device__ __forceinline__ R sv_gap(const R beta[3]) {
 template <typename R>
 struct Hencky {
     // both return whether the FP64 path was taken
-    static __device__ __forceinline__ bool stress(const R F[9], const R Fg[9], R mu, R lam, float, R tau[9]) {
-        R Fgi[9], Fe[9], beta[3], V[9];
-        hencky_eig(F, Fg, Fgi, Fe, beta, V);
+    template <typename G>
+    static __device__ __forceinline__ bool stress(const R F[9], const G& g, R mu, R lam, float, R tau[9]) {
+        R Fe[9], beta[3], V[9];
+        hencky_eig(F, g, Fe, beta, V);
         hencky_tau_from_eig(beta, V, mu, lam, tau);
         return false;
     }
-    static __device__ __forceinline__ bool vjp(const R F[9], const R Fg[9], R mu, R lam, float, const R tb[9],
+    template <typename G>
+    static __device__ __forceinline__ bool vjp(const R F[9], const G& g, R mu, R lam, float, const R tb[9],
                                                R Fb[9], R Fgb[9]) {
-        R Fgi[9], Fe[9], beta[3], V[9];
-        hencky_eig(F, Fg, Fgi, Fe, beta, V);
-        hencky_vjp_from_eig(F, Fgi, Fe, beta, V, mu, lam, tb, Fb, Fgb);
+        R Fe[9], beta[3], V[9];
+        hencky_eig(F, g, Fe, beta, V);
+        hencky_vjp_from_eig<false>(F, g, Fe, beta, V, mu, lam, tb, Fb, Fgb);
         return false;
     }
 };
@@ -393,46 +450,53 @@ struct Hencky {
 // switch).
 __device__ __forceinline__ void hencky_stress_fp64(const float F[9], const float Fg[9], float mu, float lam,
                                                    float tau[9]) {
-    double Fd[9], Fgd[9], Fgid[9], Fed[9], bd[3], Vd[9], td[9];
+    double Fd[9], Fgd[9], Fed[9], bd[3], Vd[9], td[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) { Fd[i] = F[i]; Fgd[i] = Fg[i]; }
-    hencky_eig(Fd, Fgd, Fgid, Fed, bd, Vd);
+    hencky_eig(Fd, GrowthFull<double>(Fgd), Fed, bd, Vd);
     hencky_tau_from_eig(bd, Vd, (double)mu, (double)lam, td);
 #pragma unroll
     for (int i = 0; i < 9; ++i) tau[i] = (float)td[i];
 }
 __device__ __forceinline__ void hencky_vjp_fp64(const float F[9], const float Fg[9], float mu, float lam,
                                                 const float tb[9], float Fb[9], float Fgb[9]) {
-    double Fd[9], Fgd[9], Fgid[9], Fed[9], bd[3], Vd[9], tbd[9], Fbd[9], Fgbd[9];
+    double Fd[9], Fgd[9], Fed[9], bd[3], Vd[9], tbd[9], Fbd[9], Fgbd[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) { Fd[i] = F[i]; Fgd[i] = Fg[i]; tbd[i] = tb[i]; }
-    hencky_eig(Fd, Fgd, Fgid, Fed, bd, Vd);
-    hencky_vjp_from_eig<double, true>(Fd, Fgid, Fed, bd, Vd, (double)mu, (double)lam, tbd, Fbd, Fgbd);
+    const GrowthFull<double> gd(Fgd);
+    hencky_eig(Fd, gd, Fed, bd, Vd);
+    hencky_vjp_from_eig<true>(Fd, gd, Fed, bd, Vd, (double)mu, (double)lam, tbd, Fbd, Fgbd);
 #pragma unroll
     for (int i = 0; i < 9; ++i) { Fb[i] = (float)Fbd[i]; Fgb[i] = (float)Fgbd[i]; }
 }
 
 template <>
 struct Hencky<float> {
-    static __device__ __forceinline__ bool stress(const float F[9], const float Fg[9], float mu, float lam,
+    template <typename G>
+    static __device__ __forceinline__ bool stress(const float F[9], const G& g, float mu, float lam,
                                                   float thresh, float tau[9]) {
-        float Fgi[9], Fe[9], beta[3], V[9];
-        hencky_eig(F, Fg, Fgi, Fe, beta, V);
+        float Fe[9], beta[3], V[9];
+        hencky_eig(F, g, Fe, beta, V);
         if (sv_gap(beta) >= thresh) {
             hencky_tau_from_eig(beta, V, mu, lam, tau);
             return false;
         }
+        float Fg[9];
+        g.full(Fg);
         hencky_stress_fp64(F, Fg, mu, lam, tau);
         return true;
     }
-    static __device__ __forceinline__ bool vjp(const float F[9], const float Fg[9], float mu, float lam,
+    template <typename G>
+    static __device__ __forceinline__ bool vjp(const float F[9], const G& g, float mu, float lam,
                                                float thresh, const float tb[9], float Fb[9], float Fgb[9]) {
-        float Fgi[9], Fe[9], beta[3], V[9];
-        hencky_eig(F, Fg, Fgi, Fe, beta, V);
+        float Fe[9], beta[3], V[9];
+        hencky_eig(F, g, Fe, beta, V);
         if (sv_gap(beta) >= thresh) {
-            hencky_vjp_from_eig(F, Fgi, Fe, beta, V, mu, lam, tb, Fb, Fgb);
+            hencky_vjp_from_eig<false>(F, g, Fe, beta, V, mu, lam, tb, Fb, Fgb);
             return false;
         }
+        float Fg[9];
+        g.full(Fg);
         hencky_vjp_fp64(F, Fg, mu, lam, tb, Fb, Fgb);
         return true;
     }
@@ -443,10 +507,10 @@ struct Hencky<float> {
 //   tau = kappa ln(Je) I + 2 eta(gdot) D,  D = sym(C),  gdot = sqrt(2 D:D + eps^2)
 //   eta = K gdot^(n-1) + tau_y (1 - exp(-m gdot)) / gdot
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ void hb_stress(const R F[9], const R Fg[9], const R C[9], const ModelParams<R>& P,
+template <typename R, typename G>
+__device__ __forceinline__ void hb_stress(const R F[9], const G& g, const R C[9], const ModelParams<R>& P,
                                           R tau[9]) {
-    R Je = det3(F) / det3(Fg);
+    R Je = det3(F) / g.det();
     R D[9];
     sym(C, D);
     R gdot = d_sqrt(R(2) * frob(D, D) + P.eps * P.eps);
@@ -455,15 +519,15 @@ __device__ __forceinline__ void hb_stress(const R F[9], const R Fg[9], const R C
 #pragma unroll
     for (int i = 0; i < 9; ++i) tau[i] = R(2) * eta * D[i] + ((i % 4 == 0) ? vol : R(0));
 }
-template <typename R>
-__device__ __forceinline__ void hb_vjp(const R F[9], const R Fg[9], const R C[9], const ModelParams<R>& P,
+template <typename R, typename G>
+__device__ __forceinline__ void hb_vjp(const R F[9], const G& g, const R C[9], const ModelParams<R>& P,
                                        const R tau_bar[9], R Fb[9], R Fgb[9], R Cb[9]) {
     R tb[9];
     sym(tau_bar, tb);
     R tr = tb[0] + tb[4] + tb[8];
     R Fi[9], Fgi[9];
     inv3(F, Fi);
-    inv3(Fg, Fgi);
+    g.inverse(Fgi);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -497,7 +561,7 @@ __device__ __forceinline__ void hb_vjp(const R F[9], const R Fg[9], const R C[9]
 template <typename R>
 __device__ __noinline__ bool hencky_vjp_ool(const R* F, const R* Fg, R mu, R lam, float thresh, const R* tb, R* Fb,
                                             R* Fgb) {
-    return Hencky<R>::vjp(F, Fg, mu, lam, thresh, tb, Fb, Fgb);
+    return Hencky<R>::vjp(F, GrowthFull<R>(Fg), mu, lam, thresh, tb, Fb, Fgb);
 }
 // ---------------------------------------------------------------------------
 // Hencky with the eigendecomposition kept between the stress (before the P2G
@@ -505,16 +569,20 @@ __device__ __noinline__ bool hencky_vjp_ool(const R* F, const R* Fg, R mu, R lam
 // reverse kernel.  keep = {beta[3], V[9], flag}; flag 1 means the FP32 stress
 // went to FP64 and the VJP must do the same.
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ bool hencky_stress_keep(const R* F, const R* Fg, R mu, R lam, float thresh, R* tau,
+template <typename R, typename G>
+__device__ __forceinline__ bool hencky_stress_keep(const R* F, const G& g, R mu, R lam, float thresh, R* tau,
                                                 R* keep) {
-    R Fgi[9], Fe[9], beta[3], V[9];
-    hencky_eig(F, Fg, Fgi, Fe, beta, V);
+    R Fe[9], beta[3], V[9];
+    hencky_eig(F, g, Fe, beta, V);
     bool fp64 = false;
     if constexpr (sizeof(R) == 4) fp64 = sv_gap(beta) < thresh;
     if (fp64) {
         // the FP32 solve above already failed the gap test: straight to FP64
-        if constexpr (sizeof(R) == 4) hencky_stress_fp64(F, Fg, mu, lam, tau);
+        if constexpr (sizeof(R) == 4) {
+            R Fg[9];
+            g.full(Fg);
+            hencky_stress_fp64(F, Fg, mu, lam, tau);
+        }
     } else {
         hencky_tau_from_eig(beta, V, mu, lam, tau);
     }
@@ -525,23 +593,24 @@ __device__ __forceinline__ bool hencky_stress_keep(const R* F, const R* Fg, R mu
     keep[12] = fp64 ? R(1) : R(0);
     return fp64;
 }
-template <typename R>
-__device__ __forceinline__ bool hencky_vjp_keep(const R* F, const R* Fg, R mu, R lam, float thresh, const R* tb,
+template <typename R, typename G>
+__device__ __forceinline__ bool hencky_vjp_keep(const R* F, const G& g, R mu, R lam, float thresh, const R* tb,
                                              const R* keep, R* Fb, R* Fgb) {
     if constexpr (sizeof(R) == 4) {
         if (keep[12] != R(0)) {         // the stress went to FP64: so does the VJP
+            R Fg[9];
+            g.full(Fg);
             hencky_vjp_fp64(F, Fg, mu, lam, tb, Fb, Fgb);
             return true;
         }
     }
-    R Fgi[9], Fe[9], beta[3], V[9];
-    inv3(Fg, Fgi);
-    mm(F, Fgi, Fe);
+    R Fe[9], beta[3], V[9];
+    g.elastic(F, Fe);
 #pragma unroll
     for (int i = 0; i < 3; ++i) beta[i] = keep[i];
 #pragma unroll
     for (int i = 0; i < 9; ++i) V[i] = keep[3 + i];
-    hencky_vjp_from_eig(F, Fgi, Fe, beta, V, mu, lam, tb, Fb, Fgb);
+    hencky_vjp_from_eig<false>(F, g, Fe, beta, V, mu, lam, tb, Fb, Fgb);
     return false;
 }
 
@@ -550,54 +619,47 @@ __device__ __forceinline__ bool hencky_vjp_keep(const R* F, const R* Fg, R mu, R
 // The FP32 eigensolves are inlined; the out-of-line wrappers above carry the
 // stand-alone Hencky VJP and the rare FP64 recomputes.
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ bool model_stress(const ModelParams<R>& P, float thresh, const R F[9], const R Fg[9],
+template <typename R, typename G>
+__device__ __forceinline__ bool model_stress(const ModelParams<R>& P, float thresh, const R F[9], const G& g,
                                              const R C[9], R tau[9]) {
-    if (P.kind == MPM_MODEL_HENCKY) {
-        // the eigensolve inline; only the rare FP32 -> FP64 recompute out of line
-        R Fgi[9], Fe[9], beta[3], V[9];
-        hencky_eig(F, Fg, Fgi, Fe, beta, V);
-        if constexpr (sizeof(R) == 4) {
-            if (sv_gap(beta) < thresh) {     // rare: straight to FP64, inline
-                hencky_stress_fp64(F, Fg, P.mu, P.lam, tau);
-                return true;
-            }
-        }
-        hencky_tau_from_eig(beta, V, P.mu, P.lam, tau);
-        return false;
-    }
-    if (P.kind == MPM_MODEL_HERSCHEL_BULKLEY) { hb_stress<R>(F, Fg, C, P, tau); return false; }
-    nh_stress(F, Fg, P.mu, P.lam, tau);
+    // the FP32 eigensolve and its rare FP64 recompute inline
+    if (P.kind == MPM_MODEL_HENCKY) return Hencky<R>::stress(F, g, P.mu, P.lam, thresh, tau);
+    if (P.kind == MPM_MODEL_HERSCHEL_BULKLEY) { hb_stress<R>(F, g, C, P, tau); return false; }
+    nh_stress(F, g, P.mu, P.lam, tau);
     return false;
 }
-template <typename R>
-__device__ __forceinline__ bool model_vjp(const ModelParams<R>& P, float thresh, const R F[9], const R Fg[9],
+template <typename R, typename G>
+__device__ __forceinline__ bool model_vjp(const ModelParams<R>& P, float thresh, const R F[9], const G& g,
                                           const R C[9], const R tb[9], R Fb[9], R Fgb[9], R Cb[9]) {
-    if (P.kind == MPM_MODEL_HERSCHEL_BULKLEY) { hb_vjp<R>(F, Fg, C, P, tb, Fb, Fgb, Cb); return false; }
+    if (P.kind == MPM_MODEL_HERSCHEL_BULKLEY) { hb_vjp<R>(F, g, C, P, tb, Fb, Fgb, Cb); return false; }
 #pragma unroll
     for (int i = 0; i < 9; ++i) Cb[i] = R(0);
-    if (P.kind == MPM_MODEL_HENCKY) return hencky_vjp_ool<R>(F, Fg, P.mu, P.lam, thresh, tb, Fb, Fgb);
-    nh_vjp(F, Fg, P.mu, P.lam, tb, Fb, Fgb);
+    if (P.kind == MPM_MODEL_HENCKY) {
+        R Fg[9];
+        g.full(Fg);
+        return hencky_vjp_ool<R>(F, Fg, P.mu, P.lam, thresh, tb, Fb, Fgb);
+    }
+    nh_vjp(F, g, P.mu, P.lam, tb, Fb, Fgb);
     return false;
 }
 
 // Stress and VJP for the reverse kernel, sharing Hencky's eigendecomposition.
-template <typename R>
-__device__ __forceinline__ bool model_stress_keep(const ModelParams<R>& P, float thresh, const R F[9],
-                                                  const R Fg[9], const R C[9], R tau[9], R keep[13]) {
-    if (P.kind == MPM_MODEL_HENCKY) return hencky_stress_keep<R>(F, Fg, P.mu, P.lam, thresh, tau, keep);
-    return model_stress(P, thresh, F, Fg, C, tau);
+template <typename R, typename G>
+__device__ __forceinline__ bool model_stress_keep(const ModelParams<R>& P, float thresh, const R F[9], const G& g,
+                                                  const R C[9], R tau[9], R keep[13]) {
+    if (P.kind == MPM_MODEL_HENCKY) return hencky_stress_keep<R>(F, g, P.mu, P.lam, thresh, tau, keep);
+    return model_stress(P, thresh, F, g, C, tau);
 }
-template <typename R>
-__device__ __forceinline__ bool model_vjp_keep(const ModelParams<R>& P, float thresh, const R F[9], const R Fg[9],
+template <typename R, typename G>
+__device__ __forceinline__ bool model_vjp_keep(const ModelParams<R>& P, float thresh, const R F[9], const G& g,
                                                const R C[9], const R tb[9], const R keep[13], R Fb[9], R Fgb[9],
                                                R Cb[9]) {
     if (P.kind == MPM_MODEL_HENCKY) {
 #pragma unroll
         for (int i = 0; i < 9; ++i) Cb[i] = R(0);
-        return hencky_vjp_keep<R>(F, Fg, P.mu, P.lam, thresh, tb, keep, Fb, Fgb);
+        return hencky_vjp_keep<R>(F, g, P.mu, P.lam, thresh, tb, keep, Fb, Fgb);
     }
-    return model_vjp(P, thresh, F, Fg, C, tb, Fb, Fgb, Cb);
+    return model_vjp(P, thresh, F, g, C, tb, Fb, Fgb, Cb);
 }
 
 // ---------------------------------------------------------------------------
@@ -608,16 +670,15 @@ __device__ __forceinline__ bool model_vjp_keep(const ModelParams<R>& P, float th
 // (Hencky from the eigendecomposition kept for the VJP, keep = {beta, V, flag}).
 // Herschel-Bulkley has no Lame parameters: zero.
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ void model_param_grad(const ModelParams<R>& P, const R F[9], const R Fg[9],
+template <typename R, typename G>
+__device__ __forceinline__ void model_param_grad(const ModelParams<R>& P, const R F[9], const G& g_,
                                                  const R keep[13], const R tb[9], double g[2]) {
     g[0] = 0.0;
     g[1] = 0.0;
     const R tr = tb[0] + tb[4] + tb[8];
     if (P.kind == MPM_MODEL_NEOHOOKEAN) {
-        R Fgi[9], Fe[9], b[9];
-        inv3(Fg, Fgi);
-        mm(F, Fgi, Fe);
+        R Fe[9], b[9];
+        g_.elastic(F, Fe);
         mmT(Fe, Fe, b);
         R s = 0;
 #pragma unroll

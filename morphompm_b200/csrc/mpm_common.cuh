@@ -57,8 +57,10 @@ template <typename R>
 struct SceneK {
     R dx, dt, inv_dx, pmass, vol0;
     R s_damp, mass_eps, gravity[3];     // s_damp = 1 - damping
+    R mu, lam, kappa, K, n_exp, tau_y, m_pap, eps;
+    double growth_A, ramp_steps;
     int shape[3];
-    int growth_mode;
+    int growth_mode, model;
     int wall, clamp_lo[3], clamp_hi[3];
 };
 template <typename R>
@@ -77,7 +79,18 @@ inline SceneK<R> scene_constants(const MpmScene& sc) {
         k.clamp_lo[d] = sc.clamp_lo[d];
         k.clamp_hi[d] = sc.clamp_hi[d];
     }
+    k.mu = (R)sc.mu;
+    k.lam = (R)sc.lam;
+    k.kappa = (R)sc.kappa;
+    k.K = (R)sc.K;
+    k.n_exp = (R)sc.n_exp;
+    k.tau_y = (R)sc.tau_y;
+    k.m_pap = (R)sc.m_pap;
+    k.eps = (R)sc.eps;
+    k.growth_A = sc.growth_A;
+    k.ramp_steps = sc.ramp_steps;
     k.growth_mode = sc.growth_mode;
+    k.model = sc.model;
     k.wall = sc.wall;
     return k;
 }
@@ -322,9 +335,9 @@ __device__ __forceinline__ void bspline_grad(const R fx[3], R dw[3][3]) {
 // mass and reference volume of particle p: per particle when the plan has
 // them, else the scene's
 template <typename R>
-__device__ __forceinline__ void particle_mass(const Ctx& ctx, const MpmScene& sc, long long p, R& pm, R& vol0) {
-    pm = ctx.pmass_p ? static_cast<const R*>(ctx.pmass_p)[p] : (R)sc.pmass;
-    vol0 = ctx.vol0_p ? static_cast<const R*>(ctx.vol0_p)[p] : (R)sc.vol0;
+__device__ __forceinline__ void particle_mass(const Ctx& ctx, const SceneK<R>& sc, long long p, R& pm, R& vol0) {
+    pm = ctx.pmass_p ? static_cast<const R*>(ctx.pmass_p)[p] : sc.pmass;
+    vol0 = ctx.vol0_p ? static_cast<const R*>(ctx.vol0_p)[p] : sc.vol0;
 }
 
 __device__ __forceinline__ void raise_status(int* status, int bits) {
@@ -332,7 +345,8 @@ __device__ __forceinline__ void raise_status(int* status, int bits) {
 }
 
 // Growth law g_p(t) = 1 + A * ramp(t) * phi_p (growth_mode 1)
-__device__ __forceinline__ double growth_ramp(const MpmScene& sc, int t) {
+template <typename R>
+__device__ __forceinline__ double growth_ramp(const SceneK<R>& sc, int t) {
     if (sc.ramp_steps <= 0.0) return 1.0;
     double r = (double)(t + 1) / sc.ramp_steps;
     return r < 1.0 ? r : 1.0;

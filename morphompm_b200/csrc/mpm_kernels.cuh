@@ -103,21 +103,47 @@ __device__ __forceinline__ bool node_free(const SceneK<R>& sc, int i, int j, int
     return true;
 }
 
+// The growth law's factor of particle p at step t (growth_mode 1: Fg = g I),
+// and its derivative d g / d A
+template <typename R>
+__device__ __forceinline__ R growth_factor(const Ctx& ctx, const SceneK<R>& sc, long long p, int t, R& gphi) {
+    const R phi = ctx.phi ? static_cast<const R*>(ctx.phi)[p] : R(1);
+    const double ramp = growth_ramp(sc, t);
+    gphi = (R)ramp * phi;
+    return R(1) + (R)(sc.growth_A * ramp) * phi;
+}
+
 // Fg of particle p (read, or the growth law)
 template <typename R>
-__device__ __forceinline__ void load_Fg(const Ctx& ctx, const MpmScene& sc, const MpmParticles& P, long long p,
-                                        int t, R Fg[9], R* gphi) {
+__device__ __forceinline__ void load_Fg(const Ctx& ctx, const SceneK<R>& sc, const MpmParticles& P, long long p,
+                                        int t, R Fg[9], R& gphi) {
     if (sc.growth_mode == 1) {
-        R phi = ctx.phi ? static_cast<const R*>(ctx.phi)[p] : R(1);
-        R g = R(1) + (R)(sc.growth_A * growth_ramp(sc, t)) * phi;
+        const R g = growth_factor(ctx, sc, p, t, gphi);
 #pragma unroll
         for (int i = 0; i < 9; ++i) Fg[i] = (i % 4 == 0) ? g : R(0);
-        if (gphi) *gphi = (R)growth_ramp(sc, t) * phi;
     } else {
         ld9<R>(P.Fg, p, P.sp9, P.sc9, Fg);
-        if (gphi) *gphi = R(0);
+        gphi = R(0);
     }
 }
+
+// Growth of a particle in the form a kernel is compiled for: ISO (every scene
+// of the plan follows its growth law) keeps g alone.
+template <typename R, bool ISO> struct Growth;
+template <typename R> struct Growth<R, true> {
+    GrowthIso<R> g;
+    __device__ __forceinline__ void load(const Ctx& ctx, const SceneK<R>& sc, const MpmParticles&, long long p, int t,
+                                         R& gphi) {
+        g.g = growth_factor(ctx, sc, p, t, gphi);
+    }
+};
+template <typename R> struct Growth<R, false> {
+    GrowthFull<R> g;
+    __device__ __forceinline__ void load(const Ctx& ctx, const SceneK<R>& sc, const MpmParticles& P, long long p,
+                                         int t, R& gphi) {
+        load_Fg(ctx, sc, P, p, t, g.Fg, gphi);
+    }
+};
 
 // ---------------------------------------------------------------------------
 // binning
@@ -128,7 +154,8 @@ __device__ __forceinline__ void load_Fg(const Ctx& ctx, const MpmScene& sc, cons
 // inside the grid touches (nodes base..base+2 clipped to the grid), flagged
 // where its cell key is formed.  Every particle of an occupied cell flags the
 // same tiles; the flags are plain stores of 1.
-__device__ __forceinline__ void flag_stencil_tiles(const Ctx& ctx, const MpmScene& sc, const SceneAux& ax,
+template <typename R>
+__device__ __forceinline__ void flag_stencil_tiles(const Ctx& ctx, const SceneK<R>& sc, const SceneAux& ax,
                                                    const int base[3]) {
     int tlo[3], thi[3];
 #pragma unroll
@@ -148,13 +175,14 @@ __device__ __forceinline__ void flag_stencil_tiles(const Ctx& ctx, const MpmScen
 }
 
 template <typename R>
-__device__ __forceinline__ unsigned particle_key(const Ctx& ctx, const MpmScene& sc, const SceneAux& ax,
+__device__ __forceinline__ unsigned particle_key(const Ctx& ctx, const SceneK<R>& sc, const SceneAux& ax,
                                                  const R x[3], R fx[3]) {
     int base[3];
-    const bool inside = bin_particle(x, (R)(1.0 / sc.dx), sc.shape, base, fx);
+    const bool inside = bin_particle(x, sc.inv_dx, sc.shape, base, fx);
     // the lanes of a warp in the same cell flag the same tiles: one of them does
-    const long long cell = ((long long)(base[0] + 2) * (sc.shape[1] + 2) + (base[1] + 2)) * (sc.shape[2] + 2) +
-                           (base[2] + 2);
+    // a scene's padded cells fit 32 bits; an outside particle's value is not used
+    const unsigned cell = ((unsigned)(base[0] + 2) * (unsigned)(sc.shape[1] + 2) + (unsigned)(base[1] + 2)) *
+                              (unsigned)(sc.shape[2] + 2) + (unsigned)(base[2] + 2);
     const unsigned tag = inside ? (unsigned)(ax.cell_begin + cell) : 0xffffffffu;
     const unsigned peers = __match_any_sync(__activemask(), tag);
     const bool leader = (peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0u;
@@ -174,7 +202,7 @@ bin_kernel(Ctx ctx, MpmParticles P, unsigned* __restrict__ keys) {
     int s = ctx.scene_of[p];
     R x[3], fx[3];
     ld3<R>(P.x, p, P.sp3, P.sc3, x);
-    keys[p] = particle_key<R>(ctx, ctx.scenes[s], ctx.aux[s], x, fx);
+    keys[p] = particle_key<R>(ctx, static_cast<const SceneK<R>*>(ctx.sk)[s], ctx.aux[s], x, fx);
 }
 
 // keys of a single scene (C ABI mpm_bin_keys); local keys, no plan
@@ -452,25 +480,25 @@ seg_write_kernel(Ctx ctx, const unsigned* __restrict__ skeys) {
 // forward prepass: stress -> P2G record, stored in particle order
 // record: fx[0..2], pmass, a = pmass v, B = (pmass C + dt sk) dx
 // ---------------------------------------------------------------------------
-template <typename R, int KIND = -1>
-__device__ __forceinline__ void p2g_record(const Ctx& ctx, const MpmScene& sc, long long p, const R fx[3],
-                                           const R v[3], const R C[9], const R F[9], const R Fg[9],
+template <typename R, int KIND = -1, typename G>
+__device__ __forceinline__ void p2g_record(const Ctx& ctx, const SceneK<R>& sc, long long p, const R fx[3],
+                                           const R v[3], const R C[9], const R F[9], const G& growth,
                                            R rec[PAYLOAD]) {
     ModelParams<R> M;
     M.load(sc);
     if constexpr (KIND >= 0) M.kind = KIND;     // a launch over scenes of one model
-    const R dx = (R)sc.dx, dt = (R)sc.dt, inv_dx = (R)(1.0 / sc.dx);
+    const R dx = sc.dx, dt = sc.dt, inv_dx = sc.inv_dx;
     const R k4 = R(4) * inv_dx * inv_dx;
     R tau[9];
     bool fb = false;
     if (M.kind == MPM_MODEL_EXTERNAL)
         ld9<R>(ctx.ext_tau, p, 9, 1, tau);      // the caller's stress
     else
-        fb = model_stress(M, ctx.gap_thresh, F, Fg, C, tau);
+        fb = model_stress(M, ctx.gap_thresh, F, growth, C, tau);
     if (fb) atomicAdd(ctx.fallbacks, 1ull);
     R pm, vol0;
     particle_mass<R>(ctx, sc, p, pm, vol0);
-    R c = -k4 * vol0 * det3(Fg);
+    R c = -k4 * vol0 * growth.det();
     rec[0] = fx[0]; rec[1] = fx[1]; rec[2] = fx[2]; rec[3] = pm;
 #pragma unroll
     for (int i = 0; i < 3; ++i) rec[4 + i] = pm * v[i];
@@ -484,18 +512,18 @@ __global__ void __launch_bounds__(256, 3)
 prepass_kernel(Ctx ctx, MpmParticles P, R* __restrict__ payload, int t) {
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= ctx.n) return;
-    const MpmScene& sc = ctx.scenes[ctx.scene_of[p]];
-    R x[3], v[3], C[9], F[9], Fg[9];
+    const SceneK<R>& sc = static_cast<const SceneK<R>*>(ctx.sk)[ctx.scene_of[p]];
+    R x[3], v[3], C[9], F[9], Fg[9], gphi;
     ld3<R>(P.x, p, P.sp3, P.sc3, x);
     ld3<R>(P.v, p, P.sp3, P.sc3, v);
     ld9<R>(P.C, p, P.sp9, P.sc9, C);
     ld9<R>(P.F, p, P.sp9, P.sc9, F);
-    load_Fg<R>(ctx, sc, P, p, t, Fg, nullptr);
+    load_Fg<R>(ctx, sc, P, p, t, Fg, gphi);
     int base[3];
     R fx[3];
-    bin_particle(x, (R)(1.0 / sc.dx), sc.shape, base, fx);
+    bin_particle(x, sc.inv_dx, sc.shape, base, fx);
     R rec[PAYLOAD];
-    p2g_record<R>(ctx, sc, p, fx, v, C, F, Fg, rec);
+    p2g_record<R>(ctx, sc, p, fx, v, C, F, GrowthFull<R>(Fg), rec);
     store_record(payload, p, rec);
 }
 
@@ -852,27 +880,57 @@ node_sums_kernel(Ctx ctx, const R* __restrict__ S, const int* __restrict__ activ
 
 // ---------------------------------------------------------------------------
 // stencil addressing into the dense node scratch: node (i,j,k) of a scene is
-// node_begin + (i ny + j) nz + k; per particle the three axis offsets are
-// formed once and a node costs two adds.
+// node_begin + (i ny + j) nz + k.  A particle whose 27 nodes all lie in the
+// grid takes a loop without a test per node: one address per stencil row, the
+// three nodes of a row at constant offsets.  The others (near a grid face, or
+// outside) take a rolled loop that tests every node; the choice is the
+// particle's own, so its result does not depend on its neighbours in the warp.
 // ---------------------------------------------------------------------------
-struct DenseStencil {
-    long long ox[3], oy[3];
-    int oz[3];
-    bool vx[3], vy[3], vz[3];
-    __device__ __forceinline__ void init(const MpmScene& sc, const SceneAux& ax, const int base[3]) {
-        const long long ny = sc.shape[1], nz = sc.shape[2];
-#pragma unroll
-        for (int o = 0; o < 3; ++o) {
-            const int i = base[0] + o, j = base[1] + o, k = base[2] + o;
-            vx[o] = i >= 0 && i < sc.shape[0];
-            vy[o] = j >= 0 && j < sc.shape[1];
-            vz[o] = k >= 0 && k < sc.shape[2];
-            ox[o] = ax.node_begin + (long long)i * ny * nz;
-            oy[o] = (long long)j * nz;
-            oz[o] = k;
+template <typename R>
+__device__ __forceinline__ bool stencil_interior(const SceneK<R>& sc, const int base[3]) {
+    return base[0] >= 0 && base[1] >= 0 && base[2] >= 0 && base[0] + 2 < sc.shape[0] && base[1] + 2 < sc.shape[1] &&
+           base[2] + 2 < sc.shape[2];
+}
+// Orders the loads at `at` after the computation of v: without a test per node
+// the compiler would start all 54 node loads of the reverse kernel at once and
+// spill what it holds; a third of them at a time is enough in flight (Hencky
+// 419 -> 401 us on 2.5M particles, Herschel-Bulkley 336 -> 317 on 2.1M).
+__device__ __forceinline__ void loads_after(long long& at, float& v) { asm volatile("" : "+l"(at), "+f"(v)); }
+__device__ __forceinline__ void loads_after(long long& at, double& v) { asm volatile("" : "+l"(at), "+d"(v)); }
+// weight of stencil offset o at fractional position f, and its derivative
+template <typename R>
+__device__ __forceinline__ R weight_at(int o, R f) {
+    const R a = (o == 0 ? R(1.5) : R(0.5)) - f, b = f - R(1.0);
+    return o == 1 ? R(0.75) - b * b : R(0.5) * a * a;
+}
+template <typename R>
+__device__ __forceinline__ R weight_grad_at(int o, R f) {
+    return o == 0 ? -(R(1.5) - f) : (o == 1 ? R(-2.0) * (f - R(1.0)) : f - R(0.5));
+}
+// f(offsets a, b, c, weights, node index) for every stencil node inside the grid
+template <typename R, typename Fn>
+__device__ __forceinline__ void stencil_checked(const Ctx& ctx, const SceneK<R>& sc, const SceneAux& ax,
+                                                const int base[3], const R fx[3], Fn&& f) {
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) {
+        const int i = base[0] + a;
+        if (i < 0 || i >= sc.shape[0]) continue;
+        const R wa = weight_at(a, fx[0]);
+#pragma unroll 1
+        for (int b = 0; b < 3; ++b) {
+            const int j = base[1] + b;
+            if (j < 0 || j >= sc.shape[1]) continue;
+            const R wb = weight_at(b, fx[1]);
+#pragma unroll 1
+            for (int c = 0; c < 3; ++c) {
+                const int k = base[2] + c;
+                if (k < 0 || k >= sc.shape[2]) continue;
+                const long long node = ax.node_begin + ((i * sc.shape[1] + j) * sc.shape[2] + k);
+                if (MPM_INB(node, ctx.n_nodes, 7)) f(a, b, c, wa, wb, weight_at(c, fx[2]), node);
+            }
         }
     }
-};
+}
 
 __device__ __forceinline__ void unmark_cell(const Ctx& ctx, const SceneAux& ax, const unsigned* __restrict__ skeys,
                                             long long sidx) {
@@ -887,8 +945,16 @@ __device__ __forceinline__ void unmark_cell(const Ctx& ctx, const SceneAux& ax, 
 // ---------------------------------------------------------------------------
 // Sorted slots [s_begin, s_end).  KIND >= 0: every scene of these slots uses
 // material model KIND, so the kernel carries that model's code only.
-template <typename R, bool EMIT, int KIND>
-__global__ void __launch_bounds__(256, EMIT ? (sizeof(R) == 4 ? 3 : 1) : (sizeof(R) == 4 ? 4 : 2))
+// ISO: see Growth (emitting kernels only).
+// FULL: the plan fills the GPU.  Then warps in flight count more than spills:
+// the emitting kernel at 5 CTAs per SM (48 registers) takes 154 us on 2.2M
+// neo-Hookean and 142 on 2.1M Herschel-Bulkley particles, 164 and 148 at 4, 190
+// and 174 at 3; on 4096 particles, where it waits for its own instructions and
+// loads, 3 CTAs' registers give 6.3 us and 5 CTAs' 7.7.  Hencky keeps 3: at 5
+// it would take 197 us for 222 on 2.5M, but its eigensolve is contracted
+// differently there and the FP32 results move by a rounding.
+template <typename R, bool EMIT, int KIND, bool ISO, bool FULL>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? (EMIT ? (FULL ? 5 : 3) : 4) : (EMIT && FULL ? 3 : 2))
 g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, unsigned* __restrict__ keys,
            R* __restrict__ payload, int t, long long s_begin, long long s_end) {
     long long sidx = s_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -896,52 +962,65 @@ g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, u
     long long p = tp.perm[sidx];
     if (!MPM_INB(p, ctx.n, 9)) return;
     const int s = ctx.scene_of[sidx];
-    const MpmScene& sc = ctx.scenes[s];
+    const SceneK<R>& sc = static_cast<const SceneK<R>*>(ctx.sk)[s];
     const SceneAux& ax = ctx.aux[s];
-    const R dx = (R)sc.dx, dt = (R)sc.dt, inv_dx = (R)(1.0 / sc.dx);
+    const R dx = sc.dx, dt = sc.dt, inv_dx = sc.inv_dx;
     const R k4 = R(4) * inv_dx * inv_dx;
     R x[3];
     ld3<R>(in.x, p, in.sp3, in.sc3, x);
     int base[3];
     R fx[3];
     bin_particle(x, inv_dx, sc.shape, base, fx);
-    R w[3][3];
-    bspline(fx, w);
-    DenseStencil st;
-    st.init(sc, ax, base);
     const R* __restrict__ dense = static_cast<const R*>(ctx.dense_f);
     // nC = k4 sum w g (o - fx)^T dx = k4 dx (G - nv fx^T),  G[i][d] = sum w g_i o_d
     R nv[3] = {0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (stencil_interior(sc, base)) {
+        R w[3][3];
+        bspline(fx, w);
+        const int ny = sc.shape[1], nz = sc.shape[2];
+        const long long n0 = ax.node_begin + ((base[0] * ny + base[1]) * nz + base[2]);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (!st.vx[a]) continue;
+        for (int a = 0; a < 3; ++a) {
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            if (!st.vy[b]) continue;
-            const long long rab = st.ox[a] + st.oy[b];
-            // column sums over z: sum w_c g and sum c w_c g
-            R Zg[3] = {0, 0, 0}, Zc[3] = {0, 0, 0};
+            for (int b = 0; b < 3; ++b) {
+                const long long row = n0 + (a * ny + b) * nz;
+                // column sums over z: sum w_c g and sum c w_c g
+                R Zg[3] = {0, 0, 0}, Zc[3] = {0, 0, 0};
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                if (!st.vz[c]) continue;
-                R g[4];
-                if (!MPM_INB(rab + st.oz[c], ctx.n_nodes, 7)) continue;
-                load_node(dense, rab + st.oz[c], g);
+                for (int c = 0; c < 3; ++c) {
+                    R g[4];
+                    if (!MPM_INB(row + c, ctx.n_nodes, 7)) continue;
+                    load_node(dense, row + c, g);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        Zg[i] += w[c][2] * g[1 + i];
+                        if (c) Zc[i] += (R(c) * w[c][2]) * g[1 + i];
+                    }
+                }
+                const R wab = w[a][0] * w[b][1];
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    Zg[i] += w[c][2] * g[1 + i];
-                    if (c) Zc[i] += (R(c) * w[c][2]) * g[1 + i];
+                    nv[i] += wab * Zg[i];
+                    if (a) G[3 * i + 0] += (R(a) * wab) * Zg[i];
+                    if (b) G[3 * i + 1] += (R(b) * wab) * Zg[i];
+                    G[3 * i + 2] += wab * Zc[i];
                 }
             }
-            const R wab = w[a][0] * w[b][1];
+        }
+    } else {
+        stencil_checked(ctx, sc, ax, base, fx, [&](int a, int b, int c, R wa, R wb, R wc, long long node) {
+            R g[4];
+            load_node(dense, node, g);
+            const R wt = wa * wb * wc;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                nv[i] += wab * Zg[i];
-                if (a) G[3 * i + 0] += (R(a) * wab) * Zg[i];
-                if (b) G[3 * i + 1] += (R(b) * wab) * Zg[i];
-                G[3 * i + 2] += wab * Zc[i];
+                const R q = wt * g[1 + i];
+                nv[i] += q;
+                G[3 * i + 0] += R(a) * q;
+                G[3 * i + 1] += R(b) * q;
+                G[3 * i + 2] += R(c) * q;
             }
-        }
+        });
     }
     R nC[9];
     const R kd = k4 * dx;
@@ -962,7 +1041,7 @@ g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, u
     st3<R>(out.v, p, out.sp3, out.sc3, nv);
     st9<R>(out.C, p, out.sp9, out.sc9, nC);
     st9<R>(out.F, p, out.sp9, out.sc9, Fn);
-    if (sc.growth_mode == 0 && out.Fg != nullptr && out.Fg != in.Fg) {
+    if (!ISO && sc.growth_mode == 0 && out.Fg != nullptr && out.Fg != in.Fg) {
         R Fg[9];
         ld9<R>(in.Fg, p, in.sp9, in.sc9, Fg);
         st9<R>(out.Fg, p, out.sp9, out.sc9, Fg);
@@ -973,7 +1052,7 @@ g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, u
     if constexpr (EMIT) {
         // the next step's binning and P2G record of the new state (what the
         // bin and prepass kernels of step t+1 would compute from memory)
-        R fxn[3], Fg[9], rec[PAYLOAD];
+        R fxn[3], gphi, rec[PAYLOAD];
         const unsigned kn = particle_key<R>(ctx, sc, ax, xn, fxn);
         keys[p] = kn;
         // movers of this step's sorted order (the next step's incremental re-sort)
@@ -982,8 +1061,9 @@ g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, u
             ctx.mover_flag[sidx] = moved;
             ctx.mover_pflag[p] = moved;
         }
-        load_Fg<R>(ctx, sc, in, p, t + 1, Fg, nullptr);
-        p2g_record<R, KIND>(ctx, sc, p, fxn, nv, nC, Fn, Fg, rec);
+        Growth<R, ISO> gr;
+        gr.load(ctx, sc, in, p, t + 1, gphi);
+        p2g_record<R, KIND>(ctx, sc, p, fxn, nv, nC, Fn, gr.g, rec);
         store_record(payload, p, rec);
     }
 }
@@ -998,7 +1078,13 @@ g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, u
 // MAT: also the material-parameter gradients per slot, dmat[sidx] (mu) and
 // dmat[n + sidx] (lambda).  EXT: the plan has MPM_MODEL_EXTERNAL scenes.
 // Sorted slots [s_begin, s_end); KIND as in g2p_kernel.
-template <typename R, bool MAT, bool EXT, int KIND>
+// What bounds it: instruction issue and load latency together, at 16 warps per
+// SM (128 registers; more CTAs spill and are slower).  Scene constants in the
+// plan's type, one address per stencil row without a test per node, and g
+// alone for isotropic growth cut its instructions: on 4.7M particles of two
+// models 886 -> 730 us (FP64, 0.76M: 382 -> 269), on 4096 11.0 -> 8.8.
+// ISO: see Growth, and no Fg cotangent is asked for (ib.Fg null).
+template <typename R, bool MAT, bool EXT, int KIND, bool ISO>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
 bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ outC,
                     MpmCotangents ob, MpmCotangents ib, double* __restrict__ dA, double* __restrict__ dmat,
@@ -1008,34 +1094,35 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
     long long p = tp.perm[sidx];
     if (!MPM_INB(p, ctx.n, 9)) return;
     const int s = ctx.scene_of[sidx];
-    const MpmScene& sc = ctx.scenes[s];
+    const SceneK<R>& sc = static_cast<const SceneK<R>*>(ctx.sk)[s];
     const SceneAux& ax = ctx.aux[s];
     ModelParams<R> M;
     M.load(sc);
     if constexpr (KIND >= 0) M.kind = KIND;
-    const R dx = (R)sc.dx, dt = (R)sc.dt, inv_dx = (R)(1.0 / sc.dx);
+    const R dx = sc.dx, dt = sc.dt, inv_dx = sc.inv_dx;
     const R k4 = R(4) * inv_dx * inv_dx;
     R pm, vol0;
     particle_mass<R>(ctx, sc, p, pm, vol0);
-    R x[3], C[9], F[9], Fg[9];
+    R x[3], C[9], F[9];
     R gphi;
+    Growth<R, ISO> gr;
     ld3<R>(in.x, p, in.sp3, in.sc3, x);
     ld9<R>(in.C, p, in.sp9, in.sc9, C);
     ld9<R>(in.F, p, in.sp9, in.sc9, F);
-    load_Fg<R>(ctx, sc, in, p, t, Fg, &gphi);
+    gr.load(ctx, sc, in, p, t, gphi);
 
     R tau[9], keep[13];
     bool fb = false;
     if (EXT && M.kind == MPM_MODEL_EXTERNAL)
         ld9<R>(ctx.ext_tau, p, 9, 1, tau);      // the caller's stress
     else
-        fb = model_stress_keep(M, ctx.gap_thresh, F, Fg, C, tau, keep);
+        fb = model_stress_keep(M, ctx.gap_thresh, F, gr.g, C, tau, keep);
     // the kept eigendecomposition waits in shared memory (one column per
     // thread) while the node loop holds the registers
     __shared__ R keep_s[13][256];
 #pragma unroll
     for (int i = 0; i < 13; ++i) keep_s[i][threadIdx.x] = keep[i];
-    const R c = -k4 * vol0 * det3(Fg);
+    const R c = -k4 * vol0 * gr.g.det();
 
     // per-particle matrices of the regrouped x_b terms
     R M1[9], M2[9], nvb[3], pv[3];
@@ -1051,7 +1138,10 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             nvb[i] = advect ? vnb[i] + dt * xnb[i] : vnb[i];
-            pv[i] = pm * v[i];
+            // rounded products for two components, a fused one for the third: the
+            // roundings this kernel has always had, kept whatever the compiler
+            // would contract, so that FP32 gradients stay the same bit for bit
+            pv[i] = i < 2 ? Num<R>::mul_rn(pm, v[i]) : v[i];
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 M1[3 * i + j] = k4 * (Cnb[3 * j + i] + dt * FbFt[3 * j + i]);       // k4 Cn_b'^T
@@ -1062,12 +1152,6 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
     int base[3];
     R fx[3];
     bin_particle(x, inv_dx, sc.shape, base, fx);
-    R w[3][3], dw[3][3];
-    bspline(fx, w);
-    bspline_grad(fx, dw);
-    DenseStencil st;
-    st.init(sc, ax, base);
-
     // The node loop is evaluated as separable sums: per stencil column (a,b)
     // the z-weighted sums of gv, mb and c*mb, and of the advect factor
     //   sfac(o) = gv.U(o) + mb.V(o) + pm gm_b,  U(o) = nv_b + M1^T dp, V(o) = pm v + M2^T dp
@@ -1080,67 +1164,97 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         U0[j] = nvb[j] - (D1[j] * fx[0] + D1[3 + j] * fx[1] + D1[6 + j] * fx[2]);
-        V0[j] = pv[j] - (D2[j] * fx[0] + D2[3 + j] * fx[1] + D2[6 + j] * fx[2]);
+        const R vs = D2[j] * fx[0] + D2[3 + j] * fx[1] + D2[6 + j] * fx[2];
+        V0[j] = j < 2 ? pv[j] - vs : fma(pm, pv[j], -vs);
     }
     const R* __restrict__ dfw = static_cast<const R*>(ctx.dense_f);
     const R* __restrict__ dbw = static_cast<const R*>(ctx.dense_b);
     R xs[3] = {0, 0, 0}, wgv[3] = {0, 0, 0}, wmb[3] = {0, 0, 0}, GB[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) GB[q] = R(0);
+    if (stencil_interior(sc, base)) {
+        R w[3][3], dw[3][3];
+        bspline(fx, w);
+        bspline_grad(fx, dw);
+        const int ny = sc.shape[1], nz = sc.shape[2];
+        long long n0 = ax.node_begin + ((base[0] * ny + base[1]) * nz + base[2]);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (!st.vx[a]) continue;
+        for (int a = 0; a < 3; ++a) {
+            if (a) loads_after(n0, xs[2]);
 #pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            if (!st.vy[b]) continue;
-            const long long rab = st.ox[a] + st.oy[b];
-            R Zg[3] = {0, 0, 0}, Zm[3] = {0, 0, 0}, Zc[3] = {0, 0, 0}, Sab = 0, Tab = 0;
-            R Uab[3], Vab[3];
+            for (int b = 0; b < 3; ++b) {
+                const long long row = n0 + (a * ny + b) * nz;
+                R Zg[3] = {0, 0, 0}, Zm[3] = {0, 0, 0}, Zc[3] = {0, 0, 0}, Sab = 0, Tab = 0;
+                R Uab[3], Vab[3];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                Uab[j] = U0[j] + R(a) * D1[j] + R(b) * D1[3 + j];
-                Vab[j] = V0[j] + R(a) * D2[j] + R(b) * D2[3 + j];
-            }
+                for (int j = 0; j < 3; ++j) {
+                    Uab[j] = U0[j] + R(a) * D1[j] + R(b) * D1[3 + j];
+                    Vab[j] = V0[j] + R(a) * D2[j] + R(b) * D2[3 + j];
+                }
 #pragma unroll
-            for (int cc = 0; cc < 3; ++cc) {
-                if (!st.vz[cc]) continue;
-                R gf[4], gb[4];
-                if (!MPM_INB(rab + st.oz[cc], ctx.n_nodes, 7)) continue;
-                load_node(dfw, rab + st.oz[cc], gf);
-                load_node(dbw, rab + st.oz[cc], gb);
-                const R* gv = gf + 1;
-                const R* mb = gb + 1;
-                const R wz = w[cc][2];
+                for (int cc = 0; cc < 3; ++cc) {
+                    R gf[4], gb[4];
+                    if (!MPM_INB(row + cc, ctx.n_nodes, 7)) continue;
+                    load_node(dfw, row + cc, gf);
+                    load_node(dbw, row + cc, gb);
+                    const R* gv = gf + 1;
+                    const R* mb = gb + 1;
+                    const R wz = w[cc][2];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        Zg[i] += wz * gv[i];
+                        Zm[i] += wz * mb[i];
+                        if (cc) Zc[i] += (R(cc) * wz) * mb[i];
+                    }
+                    if (advect) {
+                        R sfac = gb[0] * pm;
+#pragma unroll
+                        for (int j = 0; j < 3; ++j)
+                            sfac += gv[j] * (Uab[j] + R(cc) * D1[6 + j]) + mb[j] * (Vab[j] + R(cc) * D2[6 + j]);
+                        Sab += wz * sfac;
+                        Tab += dw[cc][2] * sfac;
+                    }
+                }
+                const R wab = w[a][0] * w[b][1];
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    Zg[i] += wz * gv[i];
-                    Zm[i] += wz * mb[i];
-                    if (cc) Zc[i] += (R(cc) * wz) * mb[i];
+                    wgv[i] += wab * Zg[i];
+                    wmb[i] += wab * Zm[i];
+                    if (a) GB[3 * i + 0] += (R(a) * wab) * Zm[i];
+                    if (b) GB[3 * i + 1] += (R(b) * wab) * Zm[i];
+                    GB[3 * i + 2] += wab * Zc[i];
                 }
                 if (advect) {
-                    R sfac = gb[0] * pm;
-#pragma unroll
-                    for (int j = 0; j < 3; ++j)
-                        sfac += gv[j] * (Uab[j] + R(cc) * D1[6 + j]) + mb[j] * (Vab[j] + R(cc) * D2[6 + j]);
-                    Sab += wz * sfac;
-                    Tab += dw[cc][2] * sfac;
+                    xs[0] += (dw[a][0] * w[b][1]) * Sab;
+                    xs[1] += (w[a][0] * dw[b][1]) * Sab;
+                    xs[2] += wab * Tab;
                 }
             }
-            const R wab = w[a][0] * w[b][1];
+        }
+    } else {
+        stencil_checked(ctx, sc, ax, base, fx, [&](int a, int b, int cc, R wa, R wb, R wc, long long node) {
+            R gf[4], gb[4];
+            load_node(dfw, node, gf);
+            load_node(dbw, node, gb);
+            const R wt = wa * wb * wc;
+            R sfac = gb[0] * pm;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                wgv[i] += wab * Zg[i];
-                wmb[i] += wab * Zm[i];
-                if (a) GB[3 * i + 0] += (R(a) * wab) * Zm[i];
-                if (b) GB[3 * i + 1] += (R(b) * wab) * Zm[i];
-                GB[3 * i + 2] += wab * Zc[i];
+                const R m = wt * gb[1 + i];
+                wgv[i] += wt * gf[1 + i];
+                wmb[i] += m;
+                GB[3 * i + 0] += R(a) * m;
+                GB[3 * i + 1] += R(b) * m;
+                GB[3 * i + 2] += R(cc) * m;
+                sfac += gf[1 + i] * (U0[i] + R(a) * D1[i] + R(b) * D1[3 + i] + R(cc) * D1[6 + i])
+                      + gb[1 + i] * (V0[i] + R(a) * D2[i] + R(b) * D2[3 + i] + R(cc) * D2[6 + i]);
             }
             if (advect) {
-                xs[0] += (dw[a][0] * w[b][1]) * Sab;
-                xs[1] += (w[a][0] * dw[b][1]) * Sab;
-                xs[2] += wab * Tab;
+                xs[0] += (weight_grad_at(a, fx[0]) * wb * wc) * sfac;
+                xs[1] += (wa * weight_grad_at(b, fx[1]) * wc) * sfac;
+                xs[2] += (wa * wb * weight_grad_at(cc, fx[2])) * sfac;
             }
-        }
+        });
     }
     R xb[3] = {xs[0] * inv_dx, xs[1] * inv_dx, xs[2] * inv_dx};
     R Sb[9];
@@ -1151,7 +1265,7 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
     // the constitutive VJP needs F, C, Fg again: reload rather than keep them live
     ld9<R>(in.C, p, in.sp9, in.sc9, C);
     ld9<R>(in.F, p, in.sp9, in.sc9, F);
-    load_Fg<R>(ctx, sc, in, p, t, Fg, &gphi);
+    gr.load(ctx, sc, in, p, t, gphi);
     R Fb[9], vb[3], Cb[9], skb[9], taub[9];
     {
         R Cn[9], Fnb[9];
@@ -1191,12 +1305,12 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
 #pragma unroll
         for (int i = 0; i < 9; ++i) Fb2[i] = Fgb[i] = Cb2[i] = R(0);
     } else {
-        fb |= model_vjp_keep(M, ctx.gap_thresh, F, Fg, C, taub, keep, Fb2, Fgb, Cb2);
+        fb |= model_vjp_keep(M, ctx.gap_thresh, F, gr.g, C, taub, keep, Fb2, Fgb, Cb2);
     }
     if (fb) atomicAdd(ctx.fallbacks, 1ull);
     if constexpr (MAT) {
         double gm[2];
-        model_param_grad(M, F, Fg, keep, taub, gm);
+        model_param_grad(M, F, gr.g, keep, taub, gm);
         dmat[sidx] = gm[0];
         dmat[ctx.n + sidx] = gm[1];
     }
@@ -1207,9 +1321,9 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
     }
     // volume path: c = -k4 vol0 det(Fg)
     R Fgi[9];
-    R dFg = inv3(Fg, Fgi);
+    R dFg = gr.g.inverse(Fgi);
     R vol = frob(skb, tau) * (-k4 * vol0) * dFg;
-    double Fgl[9];
+    double Fgl[9];      // with ISO only the diagonal is used
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -1219,7 +1333,7 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
     st3<R>(ib.v, p, ib.sp3, ib.sc3, vb);
     st9<R>(ib.C, p, ib.sp9, ib.sc9, Cb);
     st9<R>(ib.F, p, ib.sp9, ib.sc9, Fb);
-    if (ib.Fg) {
+    if (!ISO && ib.Fg) {
         double* o = ib.Fg + p * ib.sp9;
         const double* in_g = ob.Fg ? ob.Fg + p * ob.sp9 : nullptr;
 #pragma unroll
@@ -1400,7 +1514,7 @@ stress_kernel(MpmScene sc, long long n, const R* __restrict__ F, const R* __rest
 #pragma unroll
     for (int i = 0; i < 9; ++i) c[i] = R(0);
     if (KIND == MPM_MODEL_HERSCHEL_BULKLEY && C) seam_load(C, w0, n, sh, c);
-    model_stress(M, thresh, f, g, c, t);
+    model_stress(M, thresh, f, GrowthFull<R>(g), c, t);
     seam_store(tau, w0, n, sh, t);
 }
 template <typename R, int KIND>
@@ -1423,9 +1537,9 @@ stress_vjp_kernel(MpmScene sc, long long n, const R* __restrict__ F, const R* __
     for (int i = 0; i < 9; ++i) c[i] = e[i] = R(0);
     if (KIND == MPM_MODEL_HERSCHEL_BULKLEY && C) seam_load(C, w0, n, sh, c);
     if constexpr (KIND == MPM_MODEL_HENCKY)
-        Hencky<R>::vjp(f, g, M.mu, M.lam, thresh, t, a, b);
+        Hencky<R>::vjp(f, GrowthFull<R>(g), M.mu, M.lam, thresh, t, a, b);
     else
-        model_vjp(M, thresh, f, g, c, t, a, b, e);
+        model_vjp(M, thresh, f, GrowthFull<R>(g), c, t, a, b, e);
     seam_store(Fb, w0, n, sh, a);
     seam_store(Fgb, w0, n, sh, b);
     if (Cb) seam_store(Cb, w0, n, sh, e);
