@@ -281,6 +281,12 @@ int mpm_stress_vjp(const MpmScene* scene, int32_t real_bytes, int64_t n, const v
                    const void* Fg, const void* C, const void* tau_bar, void* F_bar,
                    void* Fg_bar, void* C_bar, void* stream);
 
+/* dst[r][i] = src[r][order[i]] for the rows of two (rows, n) arrays of reals
+ * (real_bytes 4 or 8): a state or cotangent slab into another particle order.
+ * No counterpart in the reference, which keeps the input order. */
+int mpm_gather_columns(const void* src, void* dst, const int32_t* order, int32_t rows, int64_t n,
+                       int32_t real_bytes, void* stream);
+
 /* Cell keys of the binning step (the stencil base of transfer.py:18-21, shifted
  * by +2 per axis and flattened over the (shape+2)^3 padded cells, z fastest;
  * particles whose stencil misses the grid get (shape+2)^3).  x is (n,3). */

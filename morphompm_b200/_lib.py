@@ -91,6 +91,7 @@ EXPORTS = {
                                   C.POINTER(MpmCotangents), vp, vp, i32, i32, vp, vp]),
     "mpm_stress": (i32, [C.POINTER(MpmScene), i32, i64, vp, vp, vp, vp, vp]),
     "mpm_stress_vjp": (i32, [C.POINTER(MpmScene), i32, i64, vp, vp, vp, vp, vp, vp, vp, vp]),
+    "mpm_gather_columns": (i32, [vp, vp, vp, i32, i64, i32, vp]),
     "mpm_bin_keys": (i32, [C.POINTER(MpmScene), i32, i64, vp, vp, vp]),
     "mpm_rollout_workspace_bytes": (i32, [vp, i32, i32, C.POINTER(C.c_size_t)]),
     "mpm_rollout_fwd": (i32, [vp, vp, vp, i32, i32, i32, vp, vp, vp]),

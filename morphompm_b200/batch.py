@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .runtime import Plan, SceneSpec, SLAB_ROWS, ROW_F, ROW_X
+from .runtime import Plan, SceneSpec, SLAB_ROWS, ROW_F, ROW_X, gather_columns
 from .trajectory import Rollout, budget_schedule, sqrt_schedule
 from .layout import batch_order
 
@@ -133,8 +133,8 @@ class Batch:
         self.order_dev = self.inverse_dev = self._stage = None
         if self.order is not None:
             dev = self.plan.device
-            self.order_dev = torch.as_tensor(self.order).to(dev)
-            self.inverse_dev = torch.as_tensor(np.argsort(self.order)).to(dev)
+            self.order_dev = torch.as_tensor(self.order.astype(np.int32)).to(dev)
+            self.inverse_dev = torch.as_tensor(np.argsort(self.order).astype(np.int32)).to(dev)
             self._stage = torch.empty(SLAB_ROWS, self.n, dtype=dtype, device=dev)
         self._copy_stream = None      # prefetch(): side-stream input copies
         self._pending = False
@@ -174,9 +174,14 @@ class Batch:
         if self.order is None:
             self.slab0.copy_(src, non_blocking=non_blocking)
         else:
-            # the caller's particle order -> the batch's cell order, on the device
-            self._stage.copy_(src, non_blocking=non_blocking)
-            torch.index_select(self._stage, 1, self.order_dev, out=self.slab0)
+            # the caller's particle order -> the batch's cell order, on the device;
+            # a slab that is there already is read where it lies
+            if not (type(src) is torch.Tensor and src.device == self._stage.device and src.dtype == self.dtype
+                    and src.shape == self._stage.shape and src.is_contiguous() and not src.is_neg()
+                    and src.untyped_storage().data_ptr() != self.slab0.untyped_storage().data_ptr()):
+                self._stage.copy_(src, non_blocking=non_blocking)
+                src = self._stage
+            gather_columns(src, self.order_dev, self.slab0)
 
     def prefetch(self, slab_host):
         """Start the host -> device copy of the next trajectory's (24, n) host
@@ -207,14 +212,14 @@ class Batch:
         if self.order is None:
             self.slab0.copy_(self._inbox)
         else:
-            torch.index_select(self._inbox, 1, self.order_dev, out=self.slab0)
+            gather_columns(self._inbox, self.order_dev, self.slab0)
         self._inbox_free.record(cur)
         self._pending = False
 
     def _to_input_order(self, slab: torch.Tensor) -> torch.Tensor:
         if self.order is None:
             return slab
-        return torch.index_select(slab, 1, self.inverse_dev)
+        return gather_columns(slab, self.inverse_dev, torch.empty_like(slab))
 
     def final_state(self) -> torch.Tensor:
         """(24, n) final state of the last trajectory, in the caller's particle order."""

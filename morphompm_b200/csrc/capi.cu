@@ -1134,15 +1134,20 @@ int mpm_rollout_fwd(MpmPlan* P, const void* state0, const void* Fg, int32_t n_st
     const size_t sb = (size_t)24 * (size_t)P->n * (size_t)P->real_bytes;
     if (L.T == 0) return async_copy(final_state, state0, sb, st);
     if (!L.recompute) {
-        // one segment: every state and tape is kept for the reverse sweep
+        // one segment: every state and tape is kept for the reverse sweep, of
+        // the final state only the C that it reads
         if ((rc = async_copy(w + L.o_seg, state0, sb, st))) return rc;
         for (int t = 0; t < L.T; ++t) {
             MpmParticles a = slab_state(P, w + L.o_seg + L.slab * t, Fg);
-            MpmParticles b = slab_state(P, w + L.o_seg + L.slab * (t + 1), Fg);
+            MpmParticles b = slab_state(P, t + 1 < L.T ? w + L.o_seg + L.slab * (t + 1) : final_state, Fg);
             rc = mpm_step_fwd_chain(P, &a, &b, advect, t, w + L.o_tape + L.tape * t, chain_flags(t, 0, L.T), st);
             if (rc) return rc;
         }
-        return async_copy(final_state, w + L.o_seg + L.slab * L.T, sb, st);
+        const size_t row = (size_t)P->n * (size_t)P->real_bytes;
+        if ((rc = async_copy(w + L.o_seg + L.slab * L.T + 6 * row, static_cast<char*>(final_state) + 6 * row, 9 * row,
+                             st)))
+            return rc;
+        return MPM_OK;
     }
     // checkpoints only; the intermediate states alternate between two scratch slabs
     if ((rc = async_copy(w + L.o_ckpt, state0, sb, st))) return rc;
@@ -1156,7 +1161,11 @@ int mpm_rollout_fwd(MpmPlan* P, const void* state0, const void* Fg, int32_t n_st
         else
             nxt = w + L.o_scr + L.slab * ((cur == w + L.o_scr + L.slab * (t % 2)) ? (t + 1) % 2 : t % 2);
         MpmParticles a = slab_state(P, cur, Fg), b = slab_state(P, nxt, Fg);
-        rc = mpm_step_fwd_chain(P, &a, &b, advect, t, nullptr, chain_flags(t, 0, L.T), st);
+        // two tapes in turn where there are two: the incremental re-sort then
+        // reads the previous order where it lies instead of copying it first
+        // (the last step's stays in the plan's scratch tape)
+        char* tape = L.k > 1 && t + 1 < L.T ? w + L.o_tape + L.tape * (t % 2) : nullptr;
+        rc = mpm_step_fwd_chain(P, &a, &b, advect, t, tape, chain_flags(t, 0, L.T), st);
         if (rc) return rc;
         cur = nxt;
     }
@@ -1183,12 +1192,13 @@ int mpm_rollout_bwd(MpmPlan* P, const void* Fg, const void* final_bar, int32_t n
     int flip = 0;
     for (int seg = L.n_seg - 1; seg >= 0; --seg) {
         const int t0 = seg * L.k, t1 = std::min(L.T, t0 + L.k);
+        // the segment's first state: its checkpoint, where there is one
+        const char* first = L.recompute ? w + L.o_ckpt + L.slab * seg : w + L.o_seg;
         if (L.recompute) {
             // the segment's states and tapes again, from its checkpoint
-            if ((rc = async_copy(w + L.o_seg, w + L.o_ckpt + L.slab * seg, sb, st))) return rc;
             for (int t = t0; t < t1; ++t) {
                 const int j = t - t0;
-                MpmParticles a = slab_state(P, w + L.o_seg + L.slab * j, Fg);
+                MpmParticles a = slab_state(P, j == 0 ? first : w + L.o_seg + L.slab * j, Fg);
                 MpmParticles b = slab_state(P, w + L.o_seg + L.slab * (j + 1), Fg);
                 rc = mpm_step_fwd_chain(P, &a, &b, advect, t, w + L.o_tape + L.tape * j, chain_flags(t, t0, t1),
                                         st);
@@ -1199,7 +1209,7 @@ int mpm_rollout_bwd(MpmPlan* P, const void* Fg, const void* final_bar, int32_t n
             const int j = t - t0;
             void* nxt = t == 0 ? state0_bar : static_cast<void*>(w + L.o_bar + L.slab * flip);
             flip ^= 1;
-            MpmParticles a = slab_state(P, w + L.o_seg + L.slab * j, Fg);
+            MpmParticles a = slab_state(P, j == 0 ? first : w + L.o_seg + L.slab * j, Fg);
             const char* outC = w + L.o_seg + L.slab * (j + 1) + (size_t)6 * P->n * P->real_bytes;
             MpmCotangents ob = slab_cot(P, cur, Fg_bar), ib = slab_cot(P, nxt, Fg_bar);
             rc = mpm_step_bwd_params(P, &a, outC, &ob, &ib, growth_grad, material_grad, advect, t,
@@ -1239,6 +1249,21 @@ int mpm_stress_vjp(const MpmScene* scene, int32_t real_bytes, int64_t n, const v
             sizeof(R) == 4 ? 1e-6f : 0.0f);
         return check_launch();
     });
+}
+
+int mpm_gather_columns(const void* src, void* dst, const int32_t* order, int32_t rows, int64_t n,
+                       int32_t real_bytes, void* stream) {
+    if (!src || !dst || !order || src == dst || rows < 0 || n < 0 || n >= (1LL << 31) ||
+        (real_bytes != 4 && real_bytes != 8))
+        return MPM_ERR_ARG;
+    if (n == 0 || rows == 0) return MPM_OK;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int g = grid_for(n, 256);
+    if (real_bytes == 4)
+        gather_columns_kernel<float><<<g, 256, 0, st>>>((const float*)src, (float*)dst, order, rows, n);
+    else
+        gather_columns_kernel<double><<<g, 256, 0, st>>>((const double*)src, (double*)dst, order, rows, n);
+    return check_launch();
 }
 
 int mpm_bin_keys(const MpmScene* scene, int32_t real_bytes, int64_t n, const void* x, int32_t* keys, void* stream) {

@@ -311,6 +311,18 @@ class Plan:
                                       C.c_void_p(stream_ptr(stream))), "mpm_loss_mse")
 
 
+def gather_columns(src: torch.Tensor, order: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """out[:, i] = src[:, order[i]] (mpm_gather_columns) on the current stream;
+    src and out (rows, n) contiguous and distinct, order int32, all on one device."""
+    assert src.is_contiguous() and out.is_contiguous() and src.shape == out.shape and src.dtype == out.dtype
+    assert order.dtype == torch.int32 and order.is_contiguous() and order.numel() == src.shape[1]
+    with torch.cuda.device(out.device):
+        L.check(L.load().mpm_gather_columns(C.c_void_p(src.data_ptr()), C.c_void_p(out.data_ptr()),
+                                            C.c_void_p(order.data_ptr()), src.shape[0], src.shape[1],
+                                            dtype_bytes(src.dtype), C.c_void_p(stream_ptr())), "mpm_gather_columns")
+    return out
+
+
 class TapeBuf:
     """Device buffer recording one forward step for its reverse."""
 

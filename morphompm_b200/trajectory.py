@@ -102,11 +102,12 @@ class Rollout:
         n = p.n
         es = self.final.element_size()
         b = self.seed_bar
-        b.zero_()
         if self.loss_kind == "detF":
+            b[:ROW_F].zero_()           # the loss kernel writes the F rows
             p.loss_detF(self.final.data_ptr() + ROW_F * n * es, 1, n, self.loss, b.data_ptr() + ROW_F * n * es,
                         stream)
         elif self.loss_kind == "mse":
+            b[ROW_X + 3:].zero_()       # and here the x rows
             p.loss_mse(self.final.data_ptr() + ROW_X * n * es, 1, n, self.x_obs.data_ptr(), self.loss,
                        b.data_ptr() + ROW_X * n * es, stream)
         else:
