@@ -127,6 +127,7 @@ Ctx make_ctx(MpmPlan* P) {
     const bool movers = P->o_mflag != SIZE_MAX && P->cs_ctas == 0;
     c.mover_flag = movers ? at<unsigned char>(P, P->o_mflag) : nullptr;
     c.mover_pflag = movers ? at<unsigned char>(P, P->o_pflag) : nullptr;
+    c.moved_count = P->cs_ctas > 0 ? at<unsigned>(P, P->o_rint) : nullptr;
     c.n = P->n;
     c.n_tiles = P->n_tiles;
     c.n_keys = P->n_keys;
@@ -445,13 +446,16 @@ int bind_cluster_sort(MpmPlan* P) {
 }
 
 // keys -> sorted order, segment table and active-tile list in one launch
-int run_cluster_sort(MpmPlan* P, const Ctx& ctx, const unsigned* keys, unsigned* skeys, unsigned* perm, int* active,
-                     int* n_active, cudaStream_t st) {
+// (old_tape: the previous step's, of a chained step, or null)
+int run_cluster_sort(MpmPlan* P, const Ctx& ctx, const unsigned* keys, const char* old_tape, unsigned* skeys,
+                     unsigned* perm, int* active, int* n_active, cudaStream_t st) {
     Site site(P, MPM_K_SORT, 1, st);
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = cluster_sort_config(P, &attr, st);
     int* flag = ctx.tile_flag;
-    void* args[] = {(void*)&ctx, (void*)&keys, (void*)&skeys, (void*)&perm, (void*)&P->cs_passes, (void*)&P->cs_bits,
+    const unsigned* ok = old_tape ? reinterpret_cast<const unsigned*>(old_tape + P->t_skeys) : nullptr;
+    const unsigned* op = old_tape ? reinterpret_cast<const unsigned*>(old_tape + P->t_perm) : nullptr;
+    void* args[] = {(void*)&ctx, (void*)&keys, (void*)&ok, (void*)&op, (void*)&skeys, (void*)&perm, (void*)&P->cs_passes, (void*)&P->cs_bits,
                     (void*)&flag, (void*)&active, (void*)&n_active};
     return cudaLaunchKernelExC(&cfg, cluster_sort_fn(P->cs_items), args) == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
@@ -472,7 +476,7 @@ int step_fwd_R(MpmPlan* P, const MpmParticles& in, MpmParticles& out, int advect
     if (!chained) { Site s(P, MPM_K_BIN, 1, st); bin_kernel<R><<<g, B, 0, st>>>(ctx, in, keys); }
     int rc;
     if (P->cs_ctas > 0) {
-        rc = run_cluster_sort(P, ctx, keys, tp.skeys, tp.perm, tp.active, tp.n_active, st);
+        rc = run_cluster_sort(P, ctx, keys, chained ? P->chain_tape : nullptr, tp.skeys, tp.perm, tp.active, tp.n_active, st);
         if (rc) return rc;
     } else {
         rc = chained && P->chain_tape && ctx.mover_flag ? run_resort(P, P->chain_tape, tape, keys, st)
@@ -881,6 +885,7 @@ int mpm_plan_bind(MpmPlan* P, void* workspace, void* stream) {
                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_status, 0, 128, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_arrived, 0, P->scenes.size() * 4, st) != cudaSuccess ||
+        cudaMemsetAsync(P->ws + P->o_rint, 0, 8, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_cell_seg, 0, (size_t)P->n_keys * 4, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_tile_flag, 0, (size_t)P->n_tiles * 4, st) != cudaSuccess)
         return MPM_ERR_CUDA;

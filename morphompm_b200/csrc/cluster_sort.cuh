@@ -6,16 +6,17 @@
 // What bounds it: latency.  A plan of a few thousand particles is sorted in
 // microseconds, but the general path (sort.cuh and the seg_* / tile_* kernels)
 // spends 14 to 24 dependent launches of 1.5 to 4 us on it.  In a captured
-// forward + adjoint trajectory this kernel takes 9.7 us for 4096 particles
-// (two 8-bit passes) and 17.6 us for 32768 (two 9-bit passes) against about
-// 46 us for those launches: 40 FP32 steps 4.23 -> 2.76 ms and 4.78 -> 3.48 ms,
-// bitwise the same results.  About a quarter of its time at 32768 is the
-// distributed-shared-memory scatter (4000 to 6000 cycles a pass).
+// forward + adjoint trajectory the passes take 9.7 us for 4096 particles (two
+// of 8 bits) and 17.6 us for 32768 (two of 9 bits) against about 46 us for
+// those launches: 40 FP32 steps 4.23 -> 2.76 ms and 4.78 -> 3.48 ms, bitwise
+// the same results.  About a quarter of that at 32768 is the scatter through
+// distributed shared memory (4000 to 6000 cycles a pass).
 #pragma once
 
 #include <cooperative_groups.h>
 
 #include "mpm_common.cuh"
+#include "sort.cuh"
 
 namespace mpm {
 
@@ -26,10 +27,11 @@ constexpr int CS_WARPS = CS_THREADS / 32;
 constexpr int CS_MAX_CTAS = 8;
 constexpr int CS_MAX_ITEMS = 8;         // keys per thread
 constexpr int CS_MAX_BITS = 10;         // digit bits per pass
+constexpr unsigned CS_MOVERS = 1024;    // particles of a merge (ranked by counting): at most CS_THREADS
 // A plan up to CS_MAX_N particles takes this path: the size the 8 CTAs hold at
 // CS_MAX_ITEMS keys per thread.  It is still the faster side there (40 FP32
-// steps of 64000 particles: 5.25 -> 4.19 ms on a 40^3 grid, 5.91 -> 4.64 ms on
-// 150^3, 55k tiles).  Its CTAs walk all tiles of the grid, hence the cap on them.
+// steps of 64000 particles, with the general path and with the passes: 5.25 and
+// 4.19 ms on a 40^3 grid, 5.91 and 4.64 ms on 150^3, 55k tiles).  Its CTAs walk all tiles of the grid, hence the cap on them.
 // The cluster takes its CTAs before a thread takes a second key (4096
 // particles: 9.7 us with 4 CTAs, 11.3 with 2, 12.9 with 1).
 constexpr long long CS_MAX_TILES = 1 << 16;
@@ -74,10 +76,17 @@ __device__ __forceinline__ unsigned cs_block_exclusive(unsigned v, unsigned* wsu
 // CTA's shared memory.  The result is the stable radix sort's: (key, particle)
 // order.  Then the segment table (as seg_write_kernel) and the active-tile
 // list (as tile_write_kernel) come from one exchange of the CTAs' counts.
+//
+// A chained step starts from the previous step's order (old_keys, old_perm;
+// null otherwise; possibly skeys and perm themselves).  When at most CS_MOVERS
+// particles changed their key, the passes are replaced by a merge, as in the
+// incremental re-sort of sort.cuh: every CTA collects all movers, ranks them by
+// (key, particle) and places the slots it owns.  32768 particles with about 160
+// movers: 13.1 us against 17.6 for two passes of 9 bits; 4096: 8.4 against 9.7.
 template <int ITEMS>
 __global__ void __launch_bounds__(CS_THREADS, 1)
-cluster_sort_kernel(Ctx ctx, const unsigned* __restrict__ keys, unsigned* __restrict__ skeys,
-                    unsigned* __restrict__ perm, int passes, int bits, int* __restrict__ tile_flag,
+cluster_sort_kernel(Ctx ctx, const unsigned* __restrict__ keys, const unsigned* old_keys, const unsigned* old_perm,
+                    unsigned* skeys, unsigned* perm, int passes, int bits, int* __restrict__ tile_flag,
                     int* __restrict__ active, int* __restrict__ n_active) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -105,6 +114,10 @@ cluster_sort_kernel(Ctx ctx, const unsigned* __restrict__ keys, unsigned* __rest
     const long long t1 = t0 + per_warp < ctx.n_tiles ? t0 + per_warp : ctx.n_tiles;
     const long long cell0 = ctx.aux[0].cell_begin, ncells = ctx.aux[0].ncells;
     unsigned k[ITEMS], v[ITEMS], rk[ITEMS];
+    // the movers that the emitting G2P counted (read by all CTAs before the
+    // first cluster barrier, set back after it)
+    const unsigned n_moved = *(volatile unsigned*)ctx.moved_count;
+    // (the passes' keys do not wait for that count)
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const long long q = q0 + i * 32;
@@ -117,7 +130,143 @@ cluster_sort_kernel(Ctx ctx, const unsigned* __restrict__ keys, unsigned* __rest
         tiles += __popc(__ballot_sync(0xffffffffu, on));
     }
 
-    for (int pass = 0; pass < passes; ++pass) {
+    const bool merged = old_keys && n_moved <= CS_MOVERS;
+    if (merged) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const long long q = q0 + i * 32;
+            k[i] = q < n ? old_keys[q] : 0xffffffffu;
+            v[i] = q < n ? old_perm[q] : 0u;
+        }
+        __shared__ unsigned long long mine_s[CS_MOVERS], all_s[CS_MOVERS], sorted_s[CS_MOVERS];
+        __shared__ unsigned mpre[CS_WARPS];
+        __shared__ unsigned cta_movers;
+        // movers of this CTA's slots, in slot order
+        unsigned moved = 0, count = 0;
+        unsigned nk[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) nk[i] = q0 + i * 32 < n && MPM_INB(v[i], n, 9) ? keys[v[i]] : k[i];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const bool mv = nk[i] != k[i];
+            moved |= (mv ? 1u : 0u) << i;
+            count += __popc(__ballot_sync(0xffffffffu, mv));
+        }
+        // the pair before each round's first slot (lane 0)
+        unsigned long long before_pair[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const long long q = q0 + i * 32;
+            before_pair[i] = lane == 0 && q > 0 && q < n ? pair_key(old_keys[q - 1], old_perm[q - 1]) : 0ull;
+        }
+        if (lane == 0) mpre[warp] = count;
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned c = mpre[lane];
+            unsigned inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            mpre[lane] = inc - c;
+            if (lane == 31) cta_movers = inc;
+        }
+        __syncthreads();
+        unsigned run = mpre[warp];               // movers of this CTA before the round
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const bool mv = (moved >> i) & 1u;
+            const unsigned ball = __ballot_sync(0xffffffffu, mv);
+            const unsigned at = run + __popc(ball & lt);
+            rk[i] = at;                          // movers of this CTA before the slot
+            if (mv && at < CS_MOVERS) mine_s[at] = pair_key(nk[i], v[i]);
+            run += __popc(ball);
+        }
+        cluster.sync();
+        unsigned m = 0, m_before = 0, first[CS_MAX_CTAS];
+#pragma unroll
+        for (int r = 0; r < CS_MAX_CTAS; ++r) {
+            const unsigned c = r < C ? *cluster.map_shared_rank(&cta_movers, r) : 0u;
+            first[r] = m;
+            m_before += r < rank ? c : 0u;
+            m += c;
+        }
+        m = m < CS_MOVERS ? m : CS_MOVERS;       // (equal to n_moved)
+        for (unsigned t = threadIdx.x; t < m; t += CS_THREADS) {
+            int owner = 0;
+            unsigned from = 0;
+#pragma unroll
+            for (int r = 1; r < CS_MAX_CTAS; ++r)
+                if (r < C && t >= first[r]) {
+                    owner = r;
+                    from = first[r];
+                }
+            all_s[t] = cluster.map_shared_rank(mine_s, owner)[t - from];
+        }
+        __syncthreads();
+        // ranks by counting, `sub` lanes to a mover: a few movers by every CTA for
+        // itself, more of them in shares that are sent to all CTAs
+        const bool split = m > CS_THREADS / 4;
+        const unsigned share = split ? (m + C - 1) / C : m;
+        unsigned sub = 32;
+        while (sub > 1 && share * sub > CS_THREADS) sub >>= 1;
+        // share * sub <= CS_THREADS: one mover per group of sub lanes
+        const unsigned part = threadIdx.x % sub, g = threadIdx.x / sub, t = (split ? rank * share : 0u) + g;
+        const bool has = g < share && t < m;
+        const unsigned long long mine = has ? all_s[t] : 0ull;
+        unsigned less = 0;
+        if (has) {
+#pragma unroll 4
+            for (unsigned j = part; j < m; j += sub) less += all_s[j] < mine ? 1u : 0u;
+        }
+        for (unsigned o = sub >> 1; o > 0; o >>= 1) less += __shfl_xor_sync(0xffffffffu, less, o);
+        if (split) {
+            if (has)
+                for (int r = (int)part; r < C; r += (int)sub) cluster.map_shared_rank(sorted_s, r)[less] = mine;
+            cluster.sync();
+        } else {
+            if (has && part == 0) sorted_s[less] = mine;
+            __syncthreads();
+        }
+        // movers ordered before the pair p
+        auto bound = [&](unsigned long long p) {
+            unsigned lo = 0, hi = m;
+            while (lo < hi) {
+                const unsigned mid = (lo + hi) >> 1;
+                if (sorted_s[mid] < p) lo = mid + 1;
+                else hi = mid;
+            }
+            return lo;
+        };
+        auto put = [&](long long pos, unsigned key, unsigned part) {
+            if (MPM_INB(pos, n, 10))
+                cluster.map_shared_rank(kv_s, (int)(pos >> SHIFT))[pos & (S - 1)] = make_uint2(key, part);
+        };
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const long long q = q0 + i * 32;
+            const unsigned b = q < n ? bound(pair_key(k[i], v[i])) : m;
+            unsigned b_prev = __shfl_up_sync(0xffffffffu, b, 1);
+            if (lane == 0) b_prev = q > 0 && q < n ? bound(before_pair[i]) : 0u;
+            if (q < n) {
+                // slots that keep their key before this one
+                const long long stay = q - (long long)(m_before + rk[i]);
+                if (!((moved >> i) & 1u)) put(stay + b, k[i], v[i]);
+                for (unsigned j = b_prev; j < b; ++j) {
+                    const unsigned long long p = sorted_s[j];
+                    put(stay + j, (unsigned)(p >> 32), (unsigned)p);
+                }
+                if (q + 1 == n)
+                    for (unsigned j = b; j < m; ++j) {
+                        const unsigned long long p = sorted_s[j];
+                        put(n - (long long)m + j, (unsigned)(p >> 32), (unsigned)p);
+                    }
+            }
+        }
+        cluster.sync();
+    }
+    for (int pass = 0; pass < (merged ? 0 : passes); ++pass) {
         const int shift = pass * bits;
         if (pass > 0) {
 #pragma unroll
@@ -272,6 +421,7 @@ cluster_sort_kernel(Ctx ctx, const unsigned* __restrict__ keys, unsigned* __rest
         tr += __popc(ball);
     }
     if (rank == 0 && threadIdx.x == 0) {
+        *ctx.moved_count = 0u;
         *ctx.n_seg = (int)seg_all;
         if (tile_all > (unsigned)ctx.active_cap) {
             raise_status(ctx.status, MPM_ERR_ARG);

@@ -119,6 +119,7 @@ struct Ctx {
     void* dense_b;               // dense node scratch, reverse record (gm_b, gmom_b[3]) per node
     unsigned char* mover_flag;   // emitting G2P: per sorted slot, its particle changed cell (may be null)
     unsigned char* mover_pflag;  // and the same flag per particle
+    unsigned* moved_count;       // cluster-sorted plans: particles whose cell the emitting G2P changed (else null)
     long long n;
     long long n_tiles;
     long long n_keys;            // padded cells of all scenes (cell_seg entries)

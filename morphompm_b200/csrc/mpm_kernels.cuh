@@ -1055,7 +1055,12 @@ g2p_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, MpmParticles out, int advect, u
         R fxn[3], gphi, rec[PAYLOAD];
         const unsigned kn = particle_key<R>(ctx, sc, ax, xn, fxn);
         keys[p] = kn;
-        // movers of this step's sorted order (the next step's incremental re-sort)
+        // movers of this step's sorted order (the next step's re-sort)
+        if (ctx.moved_count) {
+            const unsigned act = __activemask();
+            const unsigned ball = __ballot_sync(act, kn != tp.skeys[sidx]);
+            if (ball && (threadIdx.x & 31) == __ffs(act) - 1) atomicAdd(ctx.moved_count, (unsigned)__popc(ball));
+        }
         if (ctx.mover_flag) {
             const unsigned char moved = kn != tp.skeys[sidx] ? 1 : 0;
             ctx.mover_flag[sidx] = moved;

@@ -62,6 +62,48 @@ def test_sorted_order_segments_and_tiles(scenes, spread):
     plan.step_fwd(slab_particles(a), slab_particles(b), True, 0, tape)
     torch.cuda.synchronize()
 
+    _check_tape(tape, n, xs, specs)
+
+
+@pytest.mark.parametrize("scenes", [[(33, 8)], [(1024, 16)], [(4097, 32)], [(32769, 40)], [(65536, 64)],
+                                    [(700, 10), (0, 8), (1, 9), (9000, 33)]])
+@pytest.mark.parametrize("speed", [0.0, 0.0005, 0.008, 0.02, 0.5])
+def test_chained_order(scenes, speed):
+    """The order of chained steps, built from the previous step's order and the
+    particles that changed cell: none, a few, around the merge's capacity of
+    1024, and most of them (the passes)."""
+    from morphompm_b200.runtime import Plan, ROW_V, slab_particles
+    rng = np.random.default_rng(7)
+    specs, x0 = [], []
+    for n, edge in scenes:
+        dx = 1.0 / edge
+        specs.append(_scene(n, (edge, edge + 1, edge), dx))
+        x0.append(rng.uniform(0.05, 0.95, size=(n, 3)))
+    plan = Plan(specs, dtype=torch.float64)
+    n = plan.n
+    slab = np.zeros((24, n))
+    slab[0:3] = np.concatenate(x0).T
+    for i in range(3):
+        slab[15 + 4 * i] = 1.0
+    p = 0
+    for (k, edge), sp in zip(scenes, specs):
+        slab[ROW_V:ROW_V + 3, p:p + k] = rng.standard_normal((3, k)) * speed * sp.dx / sp.dt
+        p += k
+    a = torch.as_tensor(slab).cuda()
+    b = torch.empty_like(a)
+    tapes = [plan.new_tape() for _ in range(2)]
+    for t in range(4):
+        same = t == 3            # the last step overwrites the order it starts from
+        tape = tapes[(t - 1 if same else t) % 2]
+        x = a[0:3].cpu().numpy()
+        plan.step_fwd(slab_particles(a), slab_particles(b), True, t, tape, chained=t > 0, emit=t < 3)
+        torch.cuda.synchronize()
+        off = np.concatenate([[0], np.cumsum([k for k, _ in scenes])])
+        _check_tape(tape, n, [x[:, u:v].T for u, v in zip(off[:-1], off[1:])], specs)
+        a, b = b, a
+
+
+def _check_tape(tape, n, xs, specs):
     raw = tape.buf.cpu().numpy()[tape.ptr - tape.buf.data_ptr():]
     pad = lambda v: (v + 255) // 256 * 256
     at = lambda off, k: raw[off:off + 4 * k].view(np.int32).astype(np.int64)
