@@ -20,7 +20,7 @@ from typing import Optional
 
 import torch
 
-from .layout import cell_order_device
+from .layout import trajectory_order
 from .runtime import ROW_X
 from .state import ParticleState
 
@@ -62,7 +62,7 @@ class _RolloutLoss(torch.autograd.Function):
         from .transfer import get_plan, scene_spec
         p = x0.detach().contiguous()
         n = p.shape[0]
-        order = cell_order_device(p, cfg.dx, cfg.grid_shape)     # memory layout only
+        order = trajectory_order(p, cfg.dx, cfg.grid_shape)     # memory layout only
         if order is not None:
             p = p[order].contiguous()
         plan = get_plan([scene_spec(cfg, model, n)], p.dtype, p.device)

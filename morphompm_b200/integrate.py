@@ -25,7 +25,7 @@ from .runtime import SLAB_ROWS, ROW_F, ROW_X
 from .state import ParticleState
 from .constitutive import is_external
 from .config import compute_target
-from .layout import cell_order_device
+from .layout import trajectory_order
 from .transfer import get_plan, scene_spec, step, step_vjp
 
 
@@ -117,7 +117,7 @@ def dloss_dg(pts, model, cfg, g, n_steps, advect, loss: str = "detF", x_obs=None
     n = p.shape[0]
     if n == 0:
         return 0.0, 0.0     # no particles: sum det F over none
-    order = cell_order_device(p, cfg.dx, cfg.grid_shape)     # memory layout only
+    order = trajectory_order(p, cfg.dx, cfg.grid_shape)     # memory layout only
     if order is not None:
         p = p[order].contiguous()
     plan = get_plan([scene_spec(cfg, model, n)], p.dtype, p.device)
@@ -192,7 +192,7 @@ def dloss_dparams(pts, model, cfg, g, n_steps, advect, loss: str = "detF", x_obs
     n = p.shape[0]
     if n == 0:
         return 0.0, {"g": 0.0, "mu": 0.0, "lam": 0.0, "E": 0.0, "nu": 0.0}
-    order = cell_order_device(p, cfg.dx, cfg.grid_shape)     # memory layout only
+    order = trajectory_order(p, cfg.dx, cfg.grid_shape)     # memory layout only
     if order is not None:
         p = p[order].contiguous()
     plan = get_plan([scene_spec(cfg, model, n)], p.dtype, p.device)
