@@ -513,7 +513,7 @@ int step_fwd_R(MpmPlan* P, const MpmParticles& in, MpmParticles& out, int advect
             using Yes = std::true_type;
             using No = std::false_type;
             // more particles than three CTAs of 256 on every SM hold at once (FULL, see the kernel)
-            const bool full = K != MPM_MODEL_HENCKY && P->n > (long long)P->n_sm * 768;
+            const bool full = (K != MPM_MODEL_HENCKY || sizeof(R) == 8) && P->n > (long long)P->n_sm * 768;
             if (!emit) return launch(No{}, No{}, No{});
             if constexpr (K >= 0) {
                 if (P->all_growth) return full ? launch(Yes{}, Yes{}, Yes{}) : launch(Yes{}, Yes{}, No{});
@@ -582,9 +582,10 @@ int step_bwd_R(MpmPlan* P, const MpmParticles& in, const void* outC, const MpmCo
                 };
                 using Yes = std::true_type;
                 using No = std::false_type;
-                if constexpr (K == MPM_MODEL_NEOHOOKEAN || K == MPM_MODEL_HENCKY) {
+                if constexpr (K == MPM_MODEL_NEOHOOKEAN || K == MPM_MODEL_HENCKY ||
+                              (K == MPM_MODEL_HERSCHEL_BULKLEY && sizeof(R) == 8)) {
                     // every scene follows its growth law and nobody reads the Fg cotangent
-                    // (Herschel-Bulkley keeps the full form: 337 us for 317 on 2.1M particles,
+                    // (FP32 Herschel-Bulkley keeps the full form: 326 us for 317 on 2.1M particles,
                     // but the compiler contracts the short one differently and the FP32
                     // gradients move by a rounding)
                     if (P->all_growth && !ib.Fg) {

@@ -950,7 +950,7 @@ __device__ __forceinline__ void unmark_cell(const Ctx& ctx, const SceneAux& ax, 
 // the emitting kernel at 5 CTAs per SM (48 registers) takes 154 us on 2.2M
 // neo-Hookean and 142 on 2.1M Herschel-Bulkley particles, 164 and 148 at 4, 190
 // and 174 at 3; on 4096 particles, where it waits for its own instructions and
-// loads, 3 CTAs' registers give 6.3 us and 5 CTAs' 7.7.  Hencky keeps 3: at 5
+// loads, 3 CTAs' registers give 6.3 us and 5 CTAs' 7.7.  FP32 Hencky keeps 3: at 5
 // it would take 197 us for 222 on 2.5M, but its eigensolve is contracted
 // differently there and the FP32 results move by a rounding.
 template <typename R, bool EMIT, int KIND, bool ISO, bool FULL>
@@ -1153,6 +1153,14 @@ bwd_particle_kernel(Ctx ctx, Tape<R> tp, MpmParticles in, const R* __restrict__ 
                 M2[3 * i + j] = pm * C[3 * j + i] + dt * (c * tau[3 * j + i]);       // pm C^T + dt sk^T
             }
         }
+    }
+    // the new C, first read after the node loop, on its way to L2 meanwhile (rows
+    // of n: 407 -> 399 and 327 -> 322 us on 2.5M and 2.2M particles; a particle's
+    // nine values side by side gain nothing, 326 -> 338 on 1M)
+    if (in.sc9 != 1) {
+        const R* oc = outC + p * in.sp9;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) asm volatile("prefetch.global.L2 [%0];" :: "l"(oc + i * in.sc9));
     }
     int base[3];
     R fx[3];
