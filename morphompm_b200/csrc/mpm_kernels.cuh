@@ -166,12 +166,20 @@ __device__ __forceinline__ void flag_stencil_tiles(const Ctx& ctx, const SceneK<
         tlo[d] = lo >> sh;
         thi[d] = hi >> sh;
     }
-    for (int a = tlo[0]; a <= thi[0]; ++a)
-        for (int b = tlo[1]; b <= thi[1]; ++b)
-            for (int e = tlo[2]; e <= thi[2]; ++e) {
-                const long long ti = ax.tile_begin + ((long long)a * ax.ntile[1] + b) * ax.ntile[2] + e;
-                if (MPM_INB(ti, ctx.n_tiles, 1)) ctx.tile_flag[ti] = 1;
-            }
+    // three nodes lie in at most two tiles per axis (tiles have 4 nodes or more):
+    // up to eight stores, without a loop (over lo..hi per axis: binning of 4.7M
+    // particles 56 us, now 42; emitting G2P 382, now 356; with a test of the flag
+    // before the store 83 and 430)
+    const int n1 = ax.ntile[1], n2 = ax.ntile[2];
+    const long long t0 = ax.tile_begin + ((tlo[0] * n1 + tlo[1]) * n2 + tlo[2]);
+    const bool two[3] = {thi[0] > tlo[0], thi[1] > tlo[1], thi[2] > tlo[2]};
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+        const int a = o >> 2, b = (o >> 1) & 1, c = o & 1;
+        if ((a && !two[0]) || (b && !two[1]) || (c && !two[2])) continue;
+        const long long ti = t0 + ((a * n1 + b) * n2 + c);
+        if (MPM_INB(ti, ctx.n_tiles, 1)) ctx.tile_flag[ti] = 1;
+    }
 }
 
 template <typename R>
