@@ -69,8 +69,8 @@ struct MpmPlan {
     std::vector<long long> run_begin, run_end;
     bool runs_grouped = false;
     long long n_nodes = 0;
-    size_t o_dbuf, o_part, o_arrived, o_tape;     // per-slot gradients, their chunk sums, a counter per scene
-    int reduce_chunks = 1;                        // of the largest scene
+    size_t o_dbuf, o_part, o_arrived, o_chunk, o_tape;     // per-slot gradients, their chunk sums, a counter per scene
+    std::vector<SumChunk> chunks;                 // of the per-scene sums, scene by scene
     int nblk_seg = 1, nblk_tile = 1;
     // the state whose keys and P2G records the last MPM_FWD_EMIT call formed
     bool chain_valid = false;
@@ -525,18 +525,12 @@ int step_fwd_R(MpmPlan* P, const MpmParticles& in, MpmParticles& out, int advect
     return check_launch();
 }
 
-// per-scene sums of a per-slot buffer (at most 65535 scenes per launch: grid.y)
-void launch_reduce(MpmPlan* P, const Ctx& ctx, const double* v, double* out, int accumulate, int mean, int stride,
+// per-scene sums of a per-slot buffer
+void launch_reduce(MpmPlan* P, const double* v, double* out, int accumulate, int mean, int stride,
                    cudaStream_t st) {
-    const size_t S = P->scenes.size();
-    for (size_t s0 = 0; s0 < S; s0 += 65535) {
-        Ctx c = ctx;
-        c.scenes += s0;
-        const unsigned ns = (unsigned)std::min<size_t>(65535, S - s0);
-        scene_reduce_kernel<<<dim3((unsigned)P->reduce_chunks, ns), REDUCE_THREADS, 0, st>>>(
-            c, v, out + s0 * stride, at<double>(P, P->o_part) + s0 * P->reduce_chunks,
-            at<unsigned>(P, P->o_arrived) + s0, accumulate, mean, stride);
-    }
+    scene_reduce_kernel<<<(unsigned)P->chunks.size(), REDUCE_THREADS, 0, st>>>(
+        v, out, at<double>(P, P->o_part), at<unsigned>(P, P->o_arrived), at<const SumChunk>(P, P->o_chunk),
+        accumulate, mean, stride);
 }
 
 template <typename R>
@@ -601,12 +595,12 @@ int step_bwd_R(MpmPlan* P, const MpmParticles& in, const void* outC, const MpmCo
     }
     if (want_dA) {
         Site s(P, MPM_K_REDUCE, 1, st);
-        launch_reduce(P, ctx, dbuf, growth_grad, 1, 0, 1, st);
+        launch_reduce(P, dbuf, growth_grad, 1, 0, 1, st);
     }
     if (material_grad) {
         Site s(P, MPM_K_REDUCE, 2, st);
-        launch_reduce(P, ctx, dmat, material_grad, 1, 0, 2, st);
-        launch_reduce(P, ctx, dmat + P->n, material_grad + 1, 1, 0, 2, st);
+        launch_reduce(P, dmat, material_grad, 1, 0, 2, st);
+        launch_reduce(P, dmat + P->n, material_grad + 1, 1, 0, 2, st);
     }
     return check_launch();
 }
@@ -773,9 +767,13 @@ int mpm_plan_create(const MpmScene* scenes, int32_t n_scenes, int32_t real_bytes
     P->o_dense_f = L.take((size_t)P->n_nodes * 4 * R);
     P->o_dense_b = L.take((size_t)P->n_nodes * 4 * R);
     P->o_dbuf = L.take(3 * n * 8);      // dL/dA, dL/dmu, dL/dlambda per slot
-    for (const MpmScene& sc : P->scenes)
-        P->reduce_chunks = std::max(P->reduce_chunks, (int)((sc.p_end - sc.p_begin + REDUCE_CHUNK - 1) / REDUCE_CHUNK));
-    P->o_part = L.take((size_t)P->reduce_chunks * P->scenes.size() * 8);
+    for (int s = 0; s < n_scenes; ++s) {
+        const long long k = scenes[s].p_end - scenes[s].p_begin;
+        const int first = (int)P->chunks.size(), count = std::max(1, (int)((k + REDUCE_CHUNK - 1) / REDUCE_CHUNK));
+        for (int c = 0; c < count; ++c) P->chunks.push_back(SumChunk{scenes[s].p_begin, scenes[s].p_end, s, first});
+    }
+    P->o_part = L.take(P->chunks.size() * 8);
+    P->o_chunk = L.take(P->chunks.size() * sizeof(SumChunk));
     P->o_arrived = L.take(P->scenes.size() * 4);
     const size_t nw = (n + 31) / 32;
     P->nblk_resort = (int)((nw + RESORT_THREADS - 1) / RESORT_THREADS);
@@ -885,6 +883,8 @@ int mpm_plan_bind(MpmPlan* P, void* workspace, void* stream) {
         cudaMemcpyAsync(P->ws + P->o_tile_scene, P->tile_scene.data(), 4 * P->tile_scene.size(),
                         cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_status, 0, 128, st) != cudaSuccess ||
+        cudaMemcpyAsync(P->ws + P->o_chunk, P->chunks.data(), sizeof(SumChunk) * P->chunks.size(),
+                        cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_arrived, 0, P->scenes.size() * 4, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_rint, 0, 8, st) != cudaSuccess ||
         cudaMemsetAsync(P->ws + P->o_cell_seg, 0, (size_t)P->n_keys * 4, st) != cudaSuccess ||
@@ -1299,7 +1299,7 @@ int mpm_loss_detF(MpmPlan* P, const void* F, int64_t sp9, int64_t sc9, double* l
         loss_detF_kernel<float><<<g, 256, 0, st>>>(ctx, (const float*)F, sp9, sc9, dbuf, (float*)F_bar);
     else
         loss_detF_kernel<double><<<g, 256, 0, st>>>(ctx, (const double*)F, sp9, sc9, dbuf, (double*)F_bar);
-    launch_reduce(P, ctx, dbuf, loss, 0, 0, 1, st);
+    launch_reduce(P, dbuf, loss, 0, 0, 1, st);
     return check_launch();
 }
 
@@ -1317,7 +1317,7 @@ int mpm_loss_mse(MpmPlan* P, const void* x, int64_t sp3, int64_t sc3, const void
     else
         loss_mse_kernel<double><<<g, 256, 0, st>>>(ctx, (const double*)x, sp3, sc3, (const double*)x_obs, dbuf,
                                                    (double*)x_bar);
-    launch_reduce(P, ctx, dbuf, loss, 0, 1, 1, st);
+    launch_reduce(P, dbuf, loss, 0, 1, 1, st);
     return check_launch();
 }
 
