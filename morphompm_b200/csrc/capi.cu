@@ -266,8 +266,12 @@ int launch_cells(MpmPlan* P, const Ctx& ctx, const Tape<R>& tp, const R* payload
                  const MpmCotangents& ob, int advect, cudaStream_t st) {
     constexpr int W = CellSums<R>::WARPS;
     const long long blocks = std::min<long long>((P->n + W * CS_CELLS - 1) / (W * CS_CELLS), (long long)P->n_sm * 64);
-    cell_sums_kernel<R, ADJ><<<(int)std::max<long long>(1, blocks), 32 * W, 0, st>>>(
-        ctx, tp.skeys, tp.perm, payload, in, ob, at<R>(P, P->o_sums), advect);
+    auto launch = [&](auto sparse) {
+        cell_sums_kernel<R, ADJ, decltype(sparse)::value><<<(int)std::max<long long>(1, blocks), 32 * W, 0, st>>>(
+            ctx, tp.skeys, tp.perm, payload, in, ob, at<R>(P, P->o_sums), advect);
+    };
+    if (P->n > CS_SPARSE_CELLS) launch(std::true_type{});
+    else launch(std::false_type{});
     return check_launch();
 }
 

@@ -571,12 +571,12 @@ __device__ __forceinline__ void store_sum(R* __restrict__ S, long long idx, cons
 // a cell's particles were re-read from L2 (FP64: in three passes of the
 // registers' choosing).  On 4.7M FP32 particles the reverse took 284 us and the
 // forward 166, now 224 and 145; on 0.76M FP64 particles 529 and 93, now 80 and
-// 61; on 4096 FP64 particles 33 and 18, now 6.4 and 5.4.  At 4.7M it moves its
+// 61; on 4096 FP64 particles 33 and 18, now 6.4 and 5.4 (8 per cell).  At 4.7M it moves its
 // 0.95 GB (reverse) at 4.2 TB/s; the rest is the wait between a warp's loading
 // and adding (45% of the issue slots used).
 //
-// A warp takes CS_CELLS consecutive segments, whose particles are consecutive
-// sorted slots.  Its lanes first bring the particles' records into shared
+// A warp takes CS_CELLS (or 32, see CS_SPARSE_CELLS) consecutive segments, whose
+// particles are consecutive sorted slots.  Its lanes first bring the particles' records into shared
 // memory, one particle per lane (every load coalesced), at most CS_SLOTS slots
 // at a time; then three lanes per cell, one per stencil x-offset, add them up
 // in sorted order.  CS_STRIDE: reals per record in shared memory, 16 padded so
@@ -586,6 +586,19 @@ __device__ __forceinline__ void store_sum(R* __restrict__ S, long long idx, cons
 // 103 with 6, 85 with 5, and on rows of n 231 with 6, 224 with 5, 239 with 4).
 constexpr int CS_CELLS = 10;
 constexpr int CS_SLOTS = 96;
+// Cells of more slots than a window: with CS_SHARE_CELLS of them or more still to
+// be added each gets CS_SHARE places of every window, so that their lanes add
+// at the same time; fewer cells take windows of consecutive slots in turn.  FP32
+// reverse, 150 particles per cell: 32 us for 3 and 4 cells, in turn 48 and 62, for
+// 2 in turn 32; ten cells of 300 in turn took 309 us, with shares 120.
+constexpr int CS_SHARE = 8, CS_SHARE_CELLS = 3;
+// Two particles per cell or fewer leave most lanes without a record, and a
+// warp's ten cells write pieces of 160 bytes: from CS_SPARSE_CELLS cells on a warp
+// takes 32 cells, one lane each, for the three x-offsets in turn.  FP32 reverse
+// with one particle in each of 30,000 cells 6.8 us both ways, 60,000 10.4 against
+// 7.8, 400,000 70 against 44 (two per cell: 50,000 10.3 and 9.7, 15,000 5.2 and
+// 6.4; three per cell gain nothing below 100,000 cells).
+constexpr int CS_SPARSE_CELLS = 32768;
 template <typename R> struct CellSums;
 template <> struct CellSums<float>  { static constexpr int WARPS = 4, STRIDE = 20, MIN_CTAS = 5; };
 template <> struct CellSums<double> { static constexpr int WARPS = 3, STRIDE = 18, MIN_CTAS = 4; };
@@ -691,29 +704,64 @@ __device__ __forceinline__ void accumulate_record(const R r[PAYLOAD], int ox, R 
     }
 }
 
-template <typename R, bool ADJ>
-__global__ void __launch_bounds__(32 * CellSums<R>::WARPS, CellSums<R>::MIN_CTAS)
-cell_sums_kernel(Ctx ctx, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm,
-                 const R* __restrict__ payload, MpmParticles in, MpmCotangents ob, R* __restrict__ S, int advect) {
-    constexpr int W = CellSums<R>::WARPS, CH = ADJ ? 3 : 4;
-    __shared__ __align__(16) R rec_s[W][rec_at<R>(CS_SLOTS)];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    R* rec = rec_s[warp];
-    const int c = lane / 3, ox = lane % 3;
-    const int nseg = *ctx.n_seg;
-    for (int g = (blockIdx.x * W + warp) * CS_CELLS; g < nseg; g += gridDim.x * W * CS_CELLS) {
-        const int id = g + c;
-        const int cells = nseg - g < CS_CELLS ? nseg - g : CS_CELLS;
-        const bool mine = c < cells;
-        int cur = mine ? ctx.seg_first[id] : 0;
-        int last = mine ? ctx.seg_last[id] : 0;
-        if (!(MPM_INB(cur, ctx.n + 1, 11) && MPM_INB(last, ctx.n + 1, 11))) cur = last = 0;
-        if constexpr (ADJ) {
-            if (mine && ox == 0 && cur < last) {
-                const unsigned key = skeys[cur];
-                if (MPM_INB(key, ctx.n_keys, 2)) ctx.cell_seg[key] = id + 1;
+// Brings the records of the slots slot(k) < stop(k) to places 32 k + lane.
+template <typename R, bool ADJ, typename Slot, typename Stop>
+__device__ __forceinline__ void stage_records(const Ctx& ctx, const unsigned* __restrict__ perm,
+                                              const R* __restrict__ payload, const MpmParticles& in,
+                                              const MpmCotangents& ob, int advect, Slot&& slot, Stop&& stop, R* rec) {
+    const int lane = threadIdx.x & 31;
+    unsigned p[CS_SLOTS / 32];
+#pragma unroll
+    for (int k = 0; k < CS_SLOTS / 32; ++k) p[k] = slot(k) < stop(k) ? perm[slot(k)] : 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < CS_SLOTS / 32; ++k) {
+        if (slot(k) < stop(k)) {
+            R r[PAYLOAD];
+            if (!MPM_INB(p[k], ctx.n, 9)) {
+#pragma unroll
+                for (int i = 0; i < PAYLOAD; ++i) r[i] = R(0);
+            } else if constexpr (ADJ) {
+                adj_record<R>(ctx, in, ob, advect, ctx.scene_of[slot(k)], p[k], r);
+            } else {
+                load_record(payload, p[k], r);
             }
+            put_record(rec + rec_at<R>(32 * k + lane), r);
         }
+    }
+    __syncwarp();
+}
+
+// Sums of a warp's cells g .. stop - 1 (at most 32 / LANES): LANES = 3 lanes per
+// cell, one per stencil x-offset, or one lane that takes the offsets in turn.
+// With one lane the cells' records must fit one window (otherwise false, and
+// nothing is done).
+template <typename R, bool ADJ, int LANES>
+__device__ __forceinline__ bool sum_cells(const Ctx& ctx, const unsigned* __restrict__ skeys,
+                                          const unsigned* __restrict__ perm, const R* __restrict__ payload,
+                                          const MpmParticles& in, const MpmCotangents& ob, R* __restrict__ S,
+                                          int advect, int g, int stop, R* rec) {
+    constexpr int CH = ADJ ? 3 : 4;
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, c = lane / LANES, id = g + c;
+    const bool mine = c < 32 / LANES && id < stop;
+    int first = mine ? ctx.seg_first[id] : 0;
+    int last = mine ? ctx.seg_last[id] : 0;
+    if (!(MPM_INB(first, ctx.n + 1, 11) && MPM_INB(last, ctx.n + 1, 11))) first = last = 0;
+    const int end = __reduce_max_sync(ALL, last), begin = __reduce_min_sync(ALL, mine ? first : INT_MAX);
+    const bool one_window = __builtin_expect(end - begin <= CS_SLOTS, 1);
+    if (LANES == 1 && !one_window) return false;
+    if constexpr (ADJ) {
+        if (mine && lane % LANES == 0 && first < last) {
+            const unsigned key = skeys[first];
+            if (MPM_INB(key, ctx.n_keys, 2)) ctx.cell_seg[key] = id + 1;
+        }
+    }
+    if (one_window)
+        stage_records<R, ADJ>(ctx, perm, payload, in, ob, advect, [&](int k) { return begin + 32 * k + lane; },
+                              [&](int) { return end; }, rec);
+#pragma unroll 1
+    for (int pass = 0; pass < 3 / LANES; ++pass) {
+        const int ox = LANES == 3 ? lane % 3 : pass;
         R acc[3][3][CH];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
@@ -721,42 +769,39 @@ cell_sums_kernel(Ctx ctx, const unsigned* __restrict__ skeys, const unsigned* __
             for (int b = 0; b < 3; ++b)
 #pragma unroll
                 for (int h = 0; h < CH; ++h) acc[a][b][h] = R(0);
-        const int end = __reduce_max_sync(0xffffffffu, last);
-        for (;;) {
-            // the next window starts at the first slot still to be added (slots
-            // between the cells hold particles outside the grid)
-            const int w0 = __reduce_min_sync(0xffffffffu, cur < last ? cur : INT_MAX);
-            if (w0 == INT_MAX) break;
-            unsigned p[CS_SLOTS / 32];
-#pragma unroll
-            for (int k = 0; k < CS_SLOTS / 32; ++k) {
-                const int s = w0 + 32 * k + lane;
-                p[k] = s < end ? perm[s] : 0xffffffffu;
-            }
-#pragma unroll
-            for (int k = 0; k < CS_SLOTS / 32; ++k) {
-                const int s = w0 + 32 * k + lane;
-                if (s < end) {
-                    R r[PAYLOAD];
-                    if (!MPM_INB(p[k], ctx.n, 9)) {
-#pragma unroll
-                        for (int i = 0; i < PAYLOAD; ++i) r[i] = R(0);
-                    } else if constexpr (ADJ) {
-                        adj_record<R>(ctx, in, ob, advect, ctx.scene_of[s], p[k], r);
-                    } else {
-                        load_record(payload, p[k], r);
-                    }
-                    put_record(rec + rec_at<R>(32 * k + lane), r);
-                }
-            }
-            __syncwarp();
-            const int stop = last < w0 + CS_SLOTS ? last : w0 + CS_SLOTS;
-            for (; cur < stop; ++cur) {
+        // adds the records at place `at` and following, up to slot `stop`
+        auto add = [&](int& cur, int stop, int at) {
+            for (; cur < stop; ++cur, ++at) {
                 R r[PAYLOAD];
-                get_record(rec + rec_at<R>(cur - w0), r);
+                get_record(rec + rec_at<R>(at), r);
                 accumulate_record<R, ADJ>(r, ox, acc);
             }
-            __syncwarp();
+        };
+        int cur = first;
+        if (LANES == 1 || one_window) {
+            add(cur, last, cur - begin);
+        } else {
+            for (;;) {
+                // the next window starts at the first slot still to be added (slots
+                // between the cells hold particles outside the grid)
+                const int w0 = __reduce_min_sync(ALL, cur < last ? cur : INT_MAX);
+                if (w0 == INT_MAX) break;
+                // several cells that do not fit it take the same share of it each
+                const bool share = end - w0 > CS_SLOTS && __popc(__ballot_sync(ALL, cur < last)) >= 3 * CS_SHARE_CELLS;
+                int from[CS_SLOTS / 32], upto[CS_SLOTS / 32];
+#pragma unroll
+                for (int k = 0; k < CS_SLOTS / 32; ++k) {
+                    const int l = 32 * k + lane, owner = 3 * (l / CS_SHARE);    // a lane of the cell
+                    const int f = __shfl_sync(ALL, cur, owner) + l % CS_SHARE, u = __shfl_sync(ALL, last, owner);
+                    from[k] = share ? f : w0 + l;
+                    upto[k] = !share ? end : (owner < 3 * CS_CELLS ? u : 0);
+                }
+                stage_records<R, ADJ>(ctx, perm, payload, in, ob, advect, [&](int k) { return from[k]; },
+                                      [&](int k) { return upto[k]; }, rec);
+                const int upper = share ? cur + CS_SHARE : w0 + CS_SLOTS;
+                add(cur, last < upper ? last : upper, share ? CS_SHARE * c : cur - w0);
+                __syncwarp();
+            }
         }
         if (mine) {
 #pragma unroll
@@ -771,6 +816,33 @@ cell_sums_kernel(Ctx ctx, const unsigned* __restrict__ skeys, const unsigned* __
                 }
         }
     }
+    __syncwarp();       // the records are read: the warp's next cells may take their place
+    return true;
+}
+
+// SPARSE: the plan has particles enough for CS_SPARSE_CELLS cells (asked at run time,
+// the question alone costs 0.1 to 0.3 us of 4 to 6 on small plans).
+template <typename R, bool ADJ, bool SPARSE>
+__global__ void __launch_bounds__(32 * CellSums<R>::WARPS, CellSums<R>::MIN_CTAS)
+cell_sums_kernel(Ctx ctx, const unsigned* __restrict__ skeys, const unsigned* __restrict__ perm,
+                 const R* __restrict__ payload, MpmParticles in, MpmCotangents ob, R* __restrict__ S, int advect) {
+    constexpr int W = CellSums<R>::WARPS;
+    __shared__ __align__(16) R rec_s[W][rec_at<R>(CS_SLOTS)];
+    const int nseg = *ctx.n_seg, w = blockIdx.x * W + (threadIdx.x >> 5), nw = gridDim.x * W;
+    R* rec = rec_s[threadIdx.x >> 5];
+    if constexpr (SPARSE) {
+        if (nseg >= CS_SPARSE_CELLS && 2ll * nseg >= ctx.n) {
+            for (int g = w * 32; g < nseg; g += nw * 32) {
+                const int stop = nseg - g < 32 ? nseg : g + 32;
+                if (sum_cells<R, ADJ, 1>(ctx, skeys, perm, payload, in, ob, S, advect, g, stop, rec)) continue;
+                for (int h = g; h < stop; h += CS_CELLS)
+                    sum_cells<R, ADJ, 3>(ctx, skeys, perm, payload, in, ob, S, advect, h, stop, rec);
+            }
+            return;
+        }
+    }
+    for (int g = w * CS_CELLS; g < nseg; g += nw * CS_CELLS)
+        sum_cells<R, ADJ, 3>(ctx, skeys, perm, payload, in, ob, S, advect, g, nseg, rec);
 }
 
 // ---------------------------------------------------------------------------

@@ -109,3 +109,41 @@ def test_growth_law_trajectory_at_the_faces(name, dtype, shape):
                      (rows(bar, 15, 9), out[3]), (b.loss, np.array([O.loss_detF(st.F)])),
                      (b.dloss_dg, np.array([out[5]]))):
         assert _close(got, ref, tol)
+
+
+@pytest.mark.parametrize("name,dtype", [("nh", "float64"), ("hb", "float32")])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_many_sparse_cells_vs_oracle(name, dtype, shuffled):
+    """Enough cells of one or two particles for the sums to take 32 cells a warp,
+    with dense cells among them that such a warp's records do not fit."""
+    from morphompm_b200 import transfer
+    from morphompm_b200.config import Material, SimConfig
+    from morphompm_b200.state import ParticleState
+    rng = np.random.default_rng(5)
+    edge, dx = 40, 1.0 / 40
+    cells = rng.permutation(36 ** 3)[:34000]
+    counts = np.ones(len(cells), int)
+    counts[::50] = 2
+    counts[[100, 101, 5000]] = (150, 97, 400)
+    c = np.stack(np.unravel_index(np.repeat(cells, counts), (36, 36, 36)), 1) + 1
+    x = (c + 0.5 + rng.uniform(0.05, 0.95, size=c.shape)) * dx
+    if shuffled:
+        x = x[rng.permutation(len(x))]
+    n = len(x)
+    assert n <= 2 * len(cells)
+    dt = getattr(torch, dtype)
+    r = lambda *s: rng.standard_normal((n,) + s)
+    dev = [torch.as_tensor(a, dtype=dt).cuda() for a in
+           (x, 0.1 * r(3), 0.3 * r(3, 3), np.eye(3) + 0.02 * r(3, 3), 1.1 * np.eye(3) + 0.01 * r(3, 3))]
+    bars = [torch.as_tensor(a, dtype=dt).cuda() for a in (r(3), r(3), r(3, 3), r(3, 3))] + \
+           [torch.as_tensor(r(3, 3)).cuda()]
+    m, om = _models(name)
+    cfg = SimConfig(N=edge, dx=dx, dt=DT, sp=dx / 2, material=Material(E=1e3, nu=0.3))
+    scene = O.scene_from_cfg(edge, dx, DT, cfg.damping, dx / 2, cfg.material.density)
+    ns, cache = transfer.step(ParticleState(*dev), m, cfg, advect=True)
+    g = transfer.step_vjp(cache, *bars, advect=True)
+    f64 = lambda ts: [a.double().cpu().numpy() for a in ts]
+    ons, oc = O.step(O.State(*f64(dev)), om, scene, advect=True)
+    og = O.step_vjp(oc, *f64(bars), advect=True)
+    for a, b in zip((ns.x, ns.v, ns.C, ns.F, *g), (ons.x, ons.v, ons.C, ons.F, *og)):
+        assert _close(a, b, TOL[dtype])
