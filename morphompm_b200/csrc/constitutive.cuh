@@ -549,21 +549,6 @@ __device__ __forceinline__ void hb_vjp(const R F[9], const G& g, const R C[9], c
 }
 
 // ---------------------------------------------------------------------------
-// Out-of-line Hencky VJP for the run-time model switch (the stand-alone VJP
-// and the kernels over mixed or external scenes), so that its register demand
-// does not inflate the allocation of the kernels that fuse it.  The FP64
-// recompute of the stress is inline in every kernel, and so is the VJP's in
-// the model-specialised reverse kernels: out of line, such a call passes its
-// arrays through the local-memory stack and measured slower even on the rare
-// path (reverse kernel 179.3 -> 186.2 ms, G2P 93.6 -> 96.7 ms per config-4
-// trajectory).
-// ---------------------------------------------------------------------------
-template <typename R>
-__device__ __noinline__ bool hencky_vjp_ool(const R* F, const R* Fg, R mu, R lam, float thresh, const R* tb, R* Fb,
-                                            R* Fgb) {
-    return Hencky<R>::vjp(F, GrowthFull<R>(Fg), mu, lam, thresh, tb, Fb, Fgb);
-}
-// ---------------------------------------------------------------------------
 // Hencky with the eigendecomposition kept between the stress (before the P2G
 // adjoint gather) and the VJP (after it): one eigensolve per particle in the
 // reverse kernel.  keep = {beta[3], V[9], flag}; flag 1 means the FP32 stress
@@ -616,13 +601,14 @@ __device__ __forceinline__ bool hencky_vjp_keep(const R* F, const G& g, R mu, R 
 
 // ---------------------------------------------------------------------------
 // model dispatch.  Returns true when an FP32 Hencky evaluation went to FP64.
-// The FP32 eigensolves are inlined; the out-of-line wrappers above carry the
-// stand-alone Hencky VJP and the rare FP64 recomputes.
+// All of it is inline, the rare FP64 recomputes too: called out of line a VJP's
+// arrays go through the local-memory stack, slower even on the rare path
+// (reverse kernel 179.3 -> 186.2 ms, G2P 93.6 -> 96.7 per 200-step trajectory of
+// 4.5M particles).
 // ---------------------------------------------------------------------------
 template <typename R, typename G>
 __device__ __forceinline__ bool model_stress(const ModelParams<R>& P, float thresh, const R F[9], const G& g,
                                              const R C[9], R tau[9]) {
-    // the FP32 eigensolve and its rare FP64 recompute inline
     if (P.kind == MPM_MODEL_HENCKY) return Hencky<R>::stress(F, g, P.mu, P.lam, thresh, tau);
     if (P.kind == MPM_MODEL_HERSCHEL_BULKLEY) { hb_stress<R>(F, g, C, P, tau); return false; }
     nh_stress(F, g, P.mu, P.lam, tau);
@@ -634,11 +620,7 @@ __device__ __forceinline__ bool model_vjp(const ModelParams<R>& P, float thresh,
     if (P.kind == MPM_MODEL_HERSCHEL_BULKLEY) { hb_vjp<R>(F, g, C, P, tb, Fb, Fgb, Cb); return false; }
 #pragma unroll
     for (int i = 0; i < 9; ++i) Cb[i] = R(0);
-    if (P.kind == MPM_MODEL_HENCKY) {
-        R Fg[9];
-        g.full(Fg);
-        return hencky_vjp_ool<R>(F, Fg, P.mu, P.lam, thresh, tb, Fb, Fgb);
-    }
+    if (P.kind == MPM_MODEL_HENCKY) return Hencky<R>::vjp(F, g, P.mu, P.lam, thresh, tb, Fb, Fgb);
     nh_vjp(F, g, P.mu, P.lam, tb, Fb, Fgb);
     return false;
 }

@@ -1659,10 +1659,7 @@ stress_vjp_kernel(MpmScene sc, long long n, const R* __restrict__ F, const R* __
 #pragma unroll
     for (int i = 0; i < 9; ++i) c[i] = e[i] = R(0);
     if (KIND == MPM_MODEL_HERSCHEL_BULKLEY && C) seam_load(C, w0, n, sh, c);
-    if constexpr (KIND == MPM_MODEL_HENCKY)
-        Hencky<R>::vjp(f, GrowthFull<R>(g), M.mu, M.lam, thresh, t, a, b);
-    else
-        model_vjp(M, thresh, f, GrowthFull<R>(g), c, t, a, b, e);
+    model_vjp(M, thresh, f, GrowthFull<R>(g), c, t, a, b, e);
     seam_store(Fb, w0, n, sh, a);
     seam_store(Fgb, w0, n, sh, b);
     if (Cb) seam_store(Cb, w0, n, sh, e);
