@@ -326,8 +326,7 @@ def autotune(scenes: List[dict], dtype=torch.float32, steps: int = 4, budget_s: 
     the defaults) and return the fastest.  Results are deterministic whatever
     the schedule (the summation order per node does not depend on it)."""
     t_start = time.time()
-    best = {"tile_xy": 4, "tile_z": 4, "scatter_ctas_per_sm": 1, "scatter_oxb": 3 if dtype == torch.float32 else 1,
-            "particle_block": 256}
+    best = {"tile_xy": 4, "tile_z": 4, "scatter_ctas_per_sm": 1, "particle_block": 256}
     slab = torch.as_tensor(host_slab(scenes, np.float32 if dtype == torch.float32 else np.float64))
 
     def measure(cfg):
