@@ -251,14 +251,13 @@ def kernel_bytes_per_particle(kind, w):
 
 
 # DRAM bytes (read + write) per particle per launch of the heaviest kernels, from
-# `ncu` captures of a 2,092,825-particle batch of the config-4 generator (FP32,
-# chained steps; profiles/reverse_particle_dram_config4_128scenes.md and
-# profiles/forward_staged_config4_128scenes.md); their traffic grows in
-# proportion to the particles, so it is scaled to the workload.
+# `ncu` captures of these kernels on the 2,092,825 particles of the workload's
+# first 128 scenes (FP32, chained steps); their traffic grows in proportion to
+# the particles, so it is scaled to the workload.
 MEASURED_TRAFFIC_PER_PARTICLE = {
     # the neo-Hookean and the Hencky run of one step (the kernels specialised per model)
-    "bwd_particle": (281440768 + 89405440 + 244199680 + 81494016) / 2092825,
-    "g2p": (73771264 + 133358336 + 63987456 + 108095232) / 2092825,
+    "bwd_particle": (281433088 + 91372544 + 243972608 + 78332672) / 2092825,
+    "g2p": (73780992 + 132497920 + 63953920 + 107863296) / 2092825,
 }
 
 
@@ -398,8 +397,8 @@ def main():
             "unit": "GB/s", "frac": (achieved / peak) if achieved else None,
             "traffic": (MEASURED_TRAFFIC_PER_PARTICLE[dominant] * n_tot
                         if dominant in MEASURED_TRAFFIC_PER_PARTICLE else None),
-            "traffic_source": "ncu dram bytes per launch, 2.09M-particle capture scaled by particles "
-                              "(profiles/reverse_particle_dram_config4_128scenes.md)",
+            "traffic_source": "ncu dram bytes per launch of this kernel on 2.09M particles (the workload's first "
+                              "128 scenes), scaled by particles",
             "avg_launch_ms": avg_ms, "launches": nl,
             "per_launch": "one MPM step of the kernel: its launches over every material-model run of slots "
                           f"({len({sc['model'] for sc in scn if sc['x'].shape[0]})} per step) between one pair of CUDA events"}
