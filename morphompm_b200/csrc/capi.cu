@@ -247,7 +247,8 @@ template <typename R>
 int launch_nodes(MpmPlan* P, int mode, const Ctx& ctx, const int* active, const int* nact, R* grid_out,
                  const R* grid_fwd, int advect, cudaStream_t st) {
     const R* Sc = at<R>(P, P->o_sums);
-    // blocks for every node the tape's tile list can hold, at most two waves of them
+    // blocks for every node the tape's tile list can hold, at most 16 per SM and
+    // unit of the knob: two waves of the FP32 kernel, 2.7 of the FP64 one
     const long long need = ((long long)P->active_cap * P->TN + NODE_THREADS - 1) / NODE_THREADS;
     const long long room = (long long)P->n_sm * 16 * std::max(1, P->tune.scatter_ctas_per_sm);
     const int ctas = (int)std::max<long long>(1, std::min<long long>(need, room));

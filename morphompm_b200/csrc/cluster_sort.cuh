@@ -31,7 +31,10 @@ constexpr unsigned CS_MOVERS = 1024;    // particles of a merge (ranked by count
 // A plan up to CS_MAX_N particles takes this path: the size the 8 CTAs hold at
 // CS_MAX_ITEMS keys per thread.  It is still the faster side there (40 FP32
 // steps of 64000 particles, with the general path and with the passes: 5.25 and
-// 4.19 ms on a 40^3 grid, 5.91 and 4.64 ms on 150^3, 55k tiles).  Its CTAs walk all tiles of the grid, hence the cap on them.
+// 4.19 ms on a 40^3 grid, 5.91 and 4.64 ms on 150^3, 55k tiles).  Its CTAs walk
+// all tiles of the grid, hence the cap on them: with few particles, so few CTAs,
+// it is still the faster side there (forward + reverse step of 1000 FP32 particles
+// on 64,000 tiles 81 us, on 68,921 by the general path 155; 61 us on 4096 tiles).
 // The cluster takes its CTAs before a thread takes a second key (4096
 // particles: 9.7 us with 4 CTAs, 11.3 with 2, 12.9 with 1).
 constexpr long long CS_MAX_TILES = 1 << 16;

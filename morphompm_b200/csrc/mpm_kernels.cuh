@@ -148,8 +148,6 @@ template <typename R> struct Growth<R, false> {
 // ---------------------------------------------------------------------------
 // binning
 // ---------------------------------------------------------------------------
-// cell key of a particle at x (its padded stencil-base cell, or the scene's
-// "outside" key) and its fractional position fx in the stencil
 // Active tiles of the next step: the node tiles that the stencil of a particle
 // inside the grid touches (nodes base..base+2 clipped to the grid), flagged
 // where its cell key is formed.  Every particle of an occupied cell flags the
@@ -182,15 +180,18 @@ __device__ __forceinline__ void flag_stencil_tiles(const Ctx& ctx, const SceneK<
     }
 }
 
+// Cell key of a particle at x (its padded stencil-base cell, or the scene's
+// "outside" key) and its fractional position fx in the stencil; flags the tiles
+// of a particle inside.
 template <typename R>
 __device__ __forceinline__ unsigned particle_key(const Ctx& ctx, const SceneK<R>& sc, const SceneAux& ax,
                                                  const R x[3], R fx[3]) {
     int base[3];
     const bool inside = bin_particle(x, sc.inv_dx, sc.shape, base, fx);
-    // the lanes of a warp in the same cell flag the same tiles: one of them does
     // a scene's padded cells fit 32 bits; an outside particle's value is not used
     const unsigned cell = ((unsigned)(base[0] + 2) * (unsigned)(sc.shape[1] + 2) + (unsigned)(base[1] + 2)) *
                               (unsigned)(sc.shape[2] + 2) + (unsigned)(base[2] + 2);
+    // the lanes of a warp in the same cell flag the same tiles: one of them does
     const unsigned tag = inside ? (unsigned)(ax.cell_begin + cell) : 0xffffffffu;
     const unsigned peers = __match_any_sync(__activemask(), tag);
     const bool leader = (peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0u;
@@ -1587,10 +1588,10 @@ loss_mse_kernel(Ctx ctx, const R* __restrict__ x, long long sp3, long long sc3, 
 // nine coalesced rows through shared memory (a lane's own nine values lie 9
 // apart there, on distinct banks), so every sector is fetched once.  With the
 // strided loads and the out-of-line Hencky VJP, whose arrays went through the
-// local-memory stack, the pair took 215 us on 1.05M FP32 Hencky particles (37
-// stress, 167 VJP), now 110 (39 and 64: the eigensolve's instructions bound
-// both); neo-Hookean 199, now 80; Herschel-Bulkley 197, now 94; FP64 374, 268
-// and 274, now 250, 116 and 170.
+// local-memory stack, the pair took 207 us on 1.05M FP32 Hencky particles (37
+// stress, 167 VJP), now 101 (39 and 62: the eigensolve's instructions bound
+// both); neo-Hookean 192, now 71; Herschel-Bulkley 189, now 86; FP64 368, 260
+// and 266, now 241, 108 and 157.
 // ---------------------------------------------------------------------------
 constexpr int SEAM_THREADS = 128;
 template <typename R>
