@@ -316,6 +316,8 @@ def gather_columns(src: torch.Tensor, order: torch.Tensor, out: torch.Tensor) ->
     src and out (rows, n) contiguous and distinct, order int32, all on one device."""
     assert src.is_contiguous() and out.is_contiguous() and src.shape == out.shape and src.dtype == out.dtype
     assert order.dtype == torch.int32 and order.is_contiguous() and order.numel() == src.shape[1]
+    if torch.is_grad_enabled() and (src.requires_grad or out.requires_grad):
+        raise RuntimeError("gather_columns: no gradient flows through it; detach the slab first")
     with torch.cuda.device(out.device):
         L.check(L.load().mpm_gather_columns(C.c_void_p(src.data_ptr()), C.c_void_p(out.data_ptr()),
                                             C.c_void_p(order.data_ptr()), src.shape[0], src.shape[1],
